@@ -198,6 +198,7 @@ void stage_args_init(StageArgs& A, int nx, int ny, int nz, double dx, double dy,
     A.nx = nx; A.ny = ny; A.nz = nz; A.bc = bc;
     A.g = gamma; A.gm1 = gamma - 1.0;
     A.rho_floor = rho_floor; A.P_floor = P_floor; A.Pfl_gm1 = P_floor / (gamma - 1.0);
+    A.igm1 = 1.0 / (gamma - 1.0); A.gg = (gamma + 1.0) / (2.0 * gamma);
     A.idx = 1.0 / dx; A.idy = 1.0 / dy; A.idz = 1.0 / dz;
     A.dx = dx; A.dy = dy; A.dz = dz;
     A.inv2dx = 0.5 / dx; A.inv2dy = 0.5 / dy; A.inv2dz = 0.5 / dz;

@@ -462,7 +462,6 @@ struct F32Learned {
     using real = float;
     static constexpr bool kCenterFromSmem = false;
     static constexpr bool kWarpFaces = true;
-    static constexpr bool kCross = true;    // the block and all halos staged once
     static constexpr int kCols = 5;         // rho, m, P: the epilogue reloads the FP64 state
     // A sweep whose staged values all lie within a quarter of the network's
     // spread thresholds of the first one cannot hold a network row (every
@@ -485,8 +484,12 @@ struct F32Learned {
     __device__ static void floor(double (&v)[5], const f64::StageArgs& A) {
         f32::floor_screened(v, A.rho_floor, A.P_floor, A.Pfl_gm1, A.gm1);
     }
-    __device__ static void stage(double (&v)[5], bool act, const f64::StageArgs& A, float (&w)[5]) {
+    static constexpr bool kOrdinary = false;
+    __device__ static bool stage(double (&v)[5], bool act, const f64::StageArgs& A, const Consts& k, float (&w)[5],
+                                 float& P) {
         f32::stage_floored(v, act, A.rho_floor, A.P_floor, A.Pfl_gm1, A.gm1, w);
+        P = pressure(w, k);
+        return true;
     }
     __device__ static void prologue(unsigned char* psm, const f64::StageArgs& A, int nt) {
         static_assert(learned::PK_BYTES % 16 == 0, "16-byte copies of the packed parameters");

@@ -14,7 +14,6 @@ namespace tile {
 struct F32Physics {
     using real = float;
     static constexpr bool kStiffFallback = false;
-    static constexpr bool kCross = true;
     static constexpr int kCols = 5;                  // rho, m, P: the epilogue reloads the FP64 state
     static constexpr bool kCenterFromSmem = false;  // smem holds FP32 copies: reload FP64 state
     static constexpr bool kWarpFaces = false;
@@ -34,8 +33,12 @@ struct F32Physics {
     __device__ static void floor(double (&v)[5], const f64::StageArgs& A) {
         f32::floor_screened(v, A.rho_floor, A.P_floor, A.Pfl_gm1, A.gm1);
     }
-    __device__ static void stage(double (&v)[5], bool act, const f64::StageArgs& A, float (&w)[5]) {
+    static constexpr bool kOrdinary = false;
+    __device__ static bool stage(double (&v)[5], bool act, const f64::StageArgs& A, const Consts& k, float (&w)[5],
+                                 float& P) {
         f32::stage_floored(v, act, A.rho_floor, A.P_floor, A.Pfl_gm1, A.gm1, w);
+        P = pressure(w, k);
+        return true;
     }
     template <int D>
     __device__ static void flux(const float (&c)[6][6], const Consts& k, float F[5]) {

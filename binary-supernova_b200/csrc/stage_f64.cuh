@@ -45,6 +45,7 @@ struct StageArgs {
     int mode;                // 0 = RK3 stage, 1 = euler3d_rhs!
     int stage;               // 1, 2, 3
     double g, gm1, rho_floor, P_floor, Pfl_gm1;
+    double igm1, gg;         // 1 / (g - 1), (g + 1) / (2 g)
     double idx, idy, idz;
     double dt, cdt;          // cdt = 0.25*dt (stage 2), (2/3)*dt (stage 3)
     // sources

@@ -25,8 +25,6 @@ template <int TX, int TY, int TZ>
 struct Shape {
     static constexpr int T[3] = {TX, TY, TZ};
     static constexpr int NCELL = TX * TY * TZ;
-    static constexpr int EX0 = (TX + 6) * TY * TZ, EX1 = TX * (TY + 6) * TZ, EX2 = TX * TY * (TZ + 6);
-    static constexpr int NEXT = EX0 > EX1 ? (EX0 > EX2 ? EX0 : EX2) : (EX1 > EX2 ? EX1 : EX2);
     static constexpr int FC0 = (TX + 1) * TY * TZ, FC1 = TX * (TY + 1) * TZ, FC2 = TX * TY * (TZ + 1);
     static constexpr int NFACE = FC0 > FC1 ? (FC0 > FC2 ? FC0 : FC2) : (FC1 > FC2 ? FC1 : FC2);
     // "cross" staging (all three sweeps from one staged region): the block,
@@ -47,7 +45,6 @@ __host__ __device__ constexpr int pcol() { return COLS - 1; }
 struct F64Physics {
     using real = double;
     static constexpr bool kStiffFallback = false;   // (already FP64)
-    static constexpr bool kCross = true;             // stage the block and all halos once
     static constexpr bool kCenterFromSmem = true;   // smem holds the floored FP64 state
     static constexpr int kCols = 6;                 // staged columns: rho, m, E (read back by the epilogue), P
     static constexpr bool kWarpFaces = false;       // faces computed thread by thread
@@ -56,24 +53,33 @@ struct F64Physics {
     __device__ static bool same(double, double) { return true; }
     static constexpr int kExtraSmem(int) { return 0; }
     __device__ static void prologue(unsigned char*, const f64::StageArgs&, int) {}
-    struct Consts { double g, gm1; };
-    __device__ static Consts consts(const f64::StageArgs& A) { return {A.g, A.gm1}; }
+    static constexpr bool kOrdinary = true;         // faces of ordinary tiles take the shared-reciprocal code
+    struct Consts { double g, gm1, igm1, gg; bool ord; };
+    __device__ static Consts consts(const f64::StageArgs& A) {
+        const bool ok = f64::abs_hi(A.gm1) - f64::hi_pow2(-20) < f64::hi_pow2(20) - f64::hi_pow2(-20) && A.gm1 > 0.0;
+        return {A.g, A.gm1, A.igm1, A.gg, ok};
+    }
     // apply_floors (src/gpu_kernels.jl:26-46) on one cell, as the reference
     __device__ static void floor(double (&v)[5], const f64::StageArgs& A) {
-        f64::apply_floor(v[0], v[1], v[2], v[3], v[4], A.rho_floor, A.P_floor, A.Pfl_gm1, A.gm1);
+        double P;
+        f64::floor_and_pressure(v, true, A.rho_floor, A.P_floor, A.Pfl_gm1, A.gm1, &P);
     }
-    // a staged cell: floors on active cells, the staged copy
-    __device__ static void stage(double (&v)[5], bool act, const f64::StageArgs& A, double (&w)[5]) {
-        if (act) floor(v, A);
+    // a staged cell: floors on active cells, the staged copy and its
+    // pressure; whether it is ordinary (physics.cuh)
+    __device__ static bool stage(double (&v)[5], bool act, const f64::StageArgs& A, const Consts& k, double (&w)[5],
+                                 double& P) {
+        const bool ord = f64::floor_and_pressure(v, act, A.rho_floor, A.P_floor, A.Pfl_gm1, A.gm1, &P);
 #pragma unroll
         for (int q = 0; q < 5; ++q) w[q] = v[q];
-    }
-    __device__ static double pressure(const double v[5], const Consts& k) {
-        return f64::cell_pressure(v[0], v[1], v[2], v[3], v[4], k.gm1);
+        return ord;
     }
     template <int D>
     __device__ static void flux(const double (&c)[6][6], const Consts& k, double F[5]) {
-        f64::interface_flux<D>(c, k.g, k.gm1, F);
+        if (!k.ord || f64::interface_flux_ord<D>(c, k.g, k.gm1, k.igm1, k.gg, F)) general_flux<D>(c, k.g, k.gm1, F);
+    }
+    template <int D>
+    __device__ __noinline__ static void general_flux(const double (&c)[6][6], double g, double gm1, double F[5]) {
+        f64::interface_flux<D>(c, g, gm1, F);
     }
 };
 
@@ -103,7 +109,7 @@ __device__ __forceinline__ void load_cell(const f64::StageArgs& A, const Geom& G
     for (int q = 0; q < 5; ++q) v[q] = src[off + q];
 }
 
-// Staged values of the cross region (P::kCross) at entry e, from active
+// Staged values of the cross region at entry e, from active
 // coordinates (a, b, c) and the axis the cell may leave the grid along.
 template <int TX, int TY, int TZ>
 __device__ __forceinline__ void cross_cell(int e, int a0, int b0, int c0, const Geom& G, int& a, int& b, int& c,
@@ -175,73 +181,29 @@ template <class P, int TX, int TY, int TZ, int NT, int D, bool LED>
 __device__ void sweep(const f64::StageArgs& A, const Geom& G, const typename P::Consts& k, int a0, int b0, int c0,
                       typename P::real* sC, typename P::real* sF, unsigned char* psm,
                       double (&acc)[Shape<TX, TY, TZ>::NCELL / NT][5], bool quiet_cross, double* sled) {
-    constexpr bool CROSS = P::kCross;
     using S = Shape<TX, TY, TZ>;
     using real = typename P::real;
     constexpr int CPT = S::NCELL / NT;
-    constexpr int LX = TX + (D == 0 ? 6 : 0), LY = TY + (D == 1 ? 6 : 0), LZ = TZ + (D == 2 ? 6 : 0);
     constexpr int FX = TX + (D == 0), FY = TY + (D == 1), FZ = TZ + (D == 2);
-    constexpr int NE = LX * LY * LZ, NF = FX * FY * FZ;
+    constexpr int NF = FX * FY * FZ;
     constexpr int TD = D == 0 ? TX : (D == 1 ? TY : TZ);
     const int tid = threadIdx.x;
     const int n[3] = {G.nx, G.ny, G.nz};
     const int o[3] = {a0, b0, c0};
 
-    bool quiet = false;
-    if constexpr (CROSS) {
-        __syncthreads();   // staged once by stage_block; sF free after the previous sweep's divergence
-    } else {
-        __syncthreads();
-        for (int e = tid; e < NE; e += NT) {
-            int ex = e % LX, r = e / LX, ey = r % LY, ez = r / LY;
-            int a = a0 + ex - (D == 0 ? 3 : 0);
-            int b = b0 + ey - (D == 1 ? 3 : 0);
-            int c = c0 + ez - (D == 2 ? 3 : 0);
-            double v[5];
-            bool act;
-            load_cell(A, G, D, a, b, c, v, act);
-            real w[5];
-            P::stage(v, act, A, w);
-#pragma unroll
-            for (int q = 0; q < 5; ++q)
-                if (q < 4 || P::kCols == 6) sC[q * S::NEXT + e] = w[q];
-            sC[pcol<P::kCols>() * S::NEXT + e] = P::pressure(w, k);
-        }
-        // policies with per-stencil work that only non-uniform data can need
-        // (the learned weights' fallback test) learn here whether every staged
-        // value of the sweep equals the first one within the policy's margin
-        if constexpr (P::kQuiescentSkip) {
-            __syncthreads();
-            bool varied = false;
-            for (int e = tid; e < NE; e += NT) {
-#pragma unroll
-                for (int q = 0; q < 5; ++q) {   // rho, m, P (E is not reconstructed)
-                    const int col = q < 4 ? q : pcol<P::kCols>();
-                    varied |= !P::same(sC[col * S::NEXT + e], sC[col * S::NEXT]);
-                }
-            }
-            quiet = !__syncthreads_or(varied);
-        } else {
-            __syncthreads();
-        }
-    }
-    if constexpr (CROSS) quiet = quiet_cross;
-    constexpr int SD = (D == 0) ? 1 : (D == 1 ? LX : LX * LY);
-    constexpr int FSTR = CROSS ? S::NCROSS : S::NEXT;   // field stride of the staged values
+    const bool quiet = quiet_cross;
+    __syncthreads();   // staged once by stage_block; sF free after the previous sweep's divergence
+    constexpr int FSTR = S::NCROSS;   // field stride of the staged values
     // staged index of stencil cell s (0..5, cells fd-3 .. fd+2 along D) of face (fx, fy, fz)
     auto sidx = [&](int fx, int fy, int fz, int s) -> int {
-        if constexpr (!CROSS) {
-            return fx + LX * (fy + LY * fz) + s * SD;
-        } else {
-            const int fd = D == 0 ? fx : (D == 1 ? fy : fz);
-            const int p = fd - 3 + s;
-            int cb, cs, lo, hs;
-            if (D == 0) { cb = TX * (fy + TY * fz); cs = 1; lo = S::OXL + 3 * (fy + TY * fz); hs = 1; }
-            else if (D == 1) { cb = fx + TX * TY * fz; cs = TX; lo = S::OYL + fx + 3 * TX * fz; hs = TX; }
-            else { cb = fx + TX * fy; cs = TX * TY; lo = S::OZL + fx + TX * fy; hs = TX * TY; }
-            constexpr int H = D == 0 ? S::HX : (D == 1 ? S::HY : S::HZ);
-            return p < 0 ? lo + (p + 3) * hs : (p < TD ? cb + p * cs : lo + H + (p - TD) * hs);
-        }
+        const int fd = D == 0 ? fx : (D == 1 ? fy : fz);
+        const int p = fd - 3 + s;
+        int cb, cs, lo, hs;
+        if (D == 0) { cb = TX * (fy + TY * fz); cs = 1; lo = S::OXL + 3 * (fy + TY * fz); hs = 1; }
+        else if (D == 1) { cb = fx + TX * TY * fz; cs = TX; lo = S::OYL + fx + 3 * TX * fz; hs = TX; }
+        else { cb = fx + TX * fy; cs = TX * TY; lo = S::OZL + fx + TX * fy; hs = TX * TY; }
+        constexpr int H = D == 0 ? S::HX : (D == 1 ? S::HY : S::HZ);
+        return p < 0 ? lo + (p + 3) * hs : (p < TD ? cb + p * cs : lo + H + (p - TD) * hs);
     };
     // one face: write it to smem and, if this tile owns it, to the optional
     // flux arrays, coarse flux registers and fine boundary-face buffers
@@ -400,8 +362,7 @@ __device__ void sweep(const f64::StageArgs& A, const Geom& G, const typename P::
 template <class P, int TX, int TY, int TZ>
 __device__ __forceinline__ unsigned char* policy_smem(unsigned char* smem_raw) {
     using S = Shape<TX, TY, TZ>;
-    constexpr int NST = P::kCross ? S::NCROSS : S::NEXT;
-    return smem_raw + ((sizeof(typename P::real) * (P::kCols * NST + 5 * S::NFACE) + 15) / 16) * 16;
+    return smem_raw + ((sizeof(typename P::real) * (P::kCols * S::NCROSS + 5 * S::NFACE) + 15) / 16) * 16;
 }
 
 // Whether active cell (a, b, c) counts in the mass ledger: outside the
@@ -454,7 +415,7 @@ struct TmaSmem {
 // (the error word is set and the copies in flight are waited for, bounded).
 template <class P, int TX, int TY, int TZ, int NT, int MINB>
 __device__ bool stage_cross_tma(const f64::StageArgs& A, TmaCtx& T, const Geom& G, const typename P::Consts& k,
-                                int a0, int b0, int c0, typename P::real* sC) {
+                                int a0, int b0, int c0, typename P::real* sC, bool& odd) {
     using S = Shape<TX, TY, TZ>;
     using C = typename TmaSmem<P, TX, TY, TZ, NT, MINB>::C;
     using real = typename P::real;
@@ -491,12 +452,12 @@ __device__ bool stage_cross_tma(const f64::StageArgs& A, TmaCtx& T, const Geom& 
         } else {
             load_cell(A, G, d, a, b, c, v, act);
         }
-        real w[5];
-        P::stage(v, act, A, w);
+        real w[5], pr;
+        odd |= !P::stage(v, act, A, k, w, pr);
 #pragma unroll
         for (int q = 0; q < 5; ++q)
             if (q < 4 || P::kCols == 6) sC[q * S::NCROSS + e] = w[q];
-        sC[pcol<P::kCols>() * S::NCROSS + e] = P::pressure(w, k);
+        sC[pcol<P::kCols>() * S::NCROSS + e] = pr;
     };
     if (tid == 0) {
         issue(0, 0);
@@ -565,24 +526,25 @@ __device__ __forceinline__ bool stage_block(const f64::StageArgs& A, int a0, int
     static_assert(S::NCELL % NT == 0, "cells must divide evenly among threads");
     constexpr int CPT = S::NCELL / NT;
     real* sC = reinterpret_cast<real*>(smem_raw);
-    real* sF = sC + P::kCols * (P::kCross ? S::NCROSS : S::NEXT);
+    real* sF = sC + P::kCols * S::NCROSS;
 
     Geom G(A.nx, A.ny, A.nz);
     const int tid = threadIdx.x;
     if (tid == 0) nanflag = 0;
-    const typename P::Consts k = P::consts(A);
+    typename P::Consts k = P::consts(A);
+    bool odd = false;   // a staged cell outside the policy's ordinary range
     unsigned char* psm = policy_smem<P, TX, TY, TZ>(smem_raw);
     double acc[CPT][5];
     // this block's mass-ledger sums (LED kernels with A.ledger set; the other
     // kernels carry no ledger code at all)
     __shared__ double sled[LED ? f64::LED_TERMS : 1];
     if (LED && A.ledger && tid < f64::LED_TERMS) sled[tid] = 0.0;   // ordered before use by the staging barriers
-    if constexpr (P::kCross) {
+    {
         // the block and the halos of all three sweeps, staged once (floors in
         // FP64 on active cells, ghosts raw, pressure once per cell)
         __syncthreads();   // the previous block of a persistent CTA is done with smem
         if (T) {
-            if (!stage_cross_tma<P, TX, TY, TZ, NT, MINB>(A, *T, G, k, a0, b0, c0, sC)) return false;
+            if (!stage_cross_tma<P, TX, TY, TZ, NT, MINB>(A, *T, G, k, a0, b0, c0, sC, odd)) return false;
         } else {
             for (int e = tid; e < S::NCROSS; e += NT) {
                 int a, b, c, d;
@@ -590,21 +552,22 @@ __device__ __forceinline__ bool stage_block(const f64::StageArgs& A, int a0, int
                 double v[5];
                 bool act;
                 load_cell(A, G, d, a, b, c, v, act);
-                real w[5];
-                P::stage(v, act, A, w);
+                real w[5], pr;
+                odd |= !P::stage(v, act, A, k, w, pr);
 #pragma unroll
                 for (int q = 0; q < 5; ++q)
                     if (q < 4 || P::kCols == 6) sC[q * S::NCROSS + e] = w[q];
-                sC[pcol<P::kCols>() * S::NCROSS + e] = P::pressure(w, k);
+                sC[pcol<P::kCols>() * S::NCROSS + e] = pr;
             }
         }
+        if constexpr (P::kOrdinary) k.ord = !__syncthreads_or(odd || !k.ord);
     }
     // policies with per-stencil work that only non-uniform data can need (the
     // learned weights' fallback test) learn here, per sweep, whether every
     // value the sweep's stencils read (the block and that sweep's halos)
     // equals the block's first cell within the policy's margin
     bool quiet[3] = {false, false, false};
-    if constexpr (P::kCross && P::kQuiescentSkip) {
+    if constexpr (P::kQuiescentSkip) {
         __syncthreads();
         unsigned varied = 0u;   // bit 0: block, bits 1-3: x, y, z halos
         for (int e = tid; e < S::NCROSS; e += NT) {
@@ -652,9 +615,8 @@ __device__ __forceinline__ bool stage_block(const f64::StageArgs& A, int a0, int
         long long off = G.act(a, b, c);
         double u0, u1, u2, u3, u4;
         if (P::kCenterFromSmem) {
-            // the block's cells: the cross region's first part, or the z-extended block of the last sweep
-            constexpr int FS = P::kCross ? S::NCROSS : S::NEXT;
-            int e = P::kCross ? i + TX * (j + TY * kk) : i + TX * (j + TY * (kk + 3));
+            constexpr int FS = S::NCROSS;   // the block's cells: the cross region's first part
+            int e = i + TX * (j + TY * kk);
             u0 = (double)sC[0 * FS + e]; u1 = (double)sC[1 * FS + e]; u2 = (double)sC[2 * FS + e];
             u3 = (double)sC[3 * FS + e]; u4 = (double)sC[4 * FS + e];
         } else {
@@ -893,7 +855,7 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_batch(const __grid_cons
 template <class P, int TX, int TY, int TZ>
 constexpr int smem_bytes() {
     using S = Shape<TX, TY, TZ>;
-    return (P::kCols * (P::kCross ? S::NCROSS : S::NEXT) + 5 * S::NFACE) * (int)sizeof(typename P::real) + 16;
+    return (P::kCols * S::NCROSS + 5 * S::NFACE) * (int)sizeof(typename P::real) + 16;
 }
 
 // Host: launch stage_kernel_batch for the levels in B with a persistent grid
