@@ -69,14 +69,22 @@ __global__ void diag_kernel(const double* U, int nx, int ny, int nz, double dx, 
 }
 
 // totals times dV -> out[0..NDIAG); with the device loop's counters, the
-// record {t, dt, totals} at index steps - 1 when it is below cap.
+// record {t, dt, totals} at index steps - 1 when it is below cap.  A warp per
+// total: its lanes merge every 32nd partial, then one another in a fixed tree,
+// so the result does not depend on scheduling.  (One thread per total walked
+// the partials' loads in a chain: 70 us, against 6 us.)
 __global__ void diag_finish(const double* part, int nblocks, double dV, double* out, const double* t,
                             const double* dt, const int* steps, const int* done, int cap, const double* ledger) {
     if (done && *done) return;
-    const int q = threadIdx.x;
+    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (q >= NDIAG || blockIdx.x != 0) return;
     DD acc = {0.0, 0.0};
-    for (int b = 0; b < nblocks; ++b) acc = dd_merge(acc, DD{part[2 * (NDIAG * b + q)], part[2 * (NDIAG * b + q) + 1]});
+#pragma unroll 4
+    for (int b = lane; b < nblocks; b += 32)
+        acc = dd_merge(acc, DD{part[2 * (NDIAG * b + q)], part[2 * (NDIAG * b + q) + 1]});
+    for (int o = 16; o > 0; o >>= 1)
+        acc = dd_merge(acc, DD{__shfl_xor_sync(0xffffffffu, acc.hi, o), __shfl_xor_sync(0xffffffffu, acc.lo, o)});
+    if (lane) return;
     double v = (acc.hi + acc.lo) * dV;
     if (!steps) { out[q] = v; return; }
     const int k = *steps - 1;
@@ -95,7 +103,7 @@ bsn_status launch(bsn_ctx* ctx, const double* U, int nx, int ny, int nz, double 
     diag_kernel<<<BLOCKS, 256, 0, ctx->stream>>>(U, nx, ny, nz, dx, dy, dz, x0, y0, z0, bhs_dev, nbh_dev, nbh, gamma,
                                                  done, part);
     BSN_TRY(launch_check(ctx, "diag_kernel"));
-    diag_finish<<<1, 32, 0, ctx->stream>>>(part, BLOCKS, dx * dy * dz, out, t, dt, steps, done, cap, ledger);
+    diag_finish<<<1, 32 * NDIAG, 0, ctx->stream>>>(part, BLOCKS, dx * dy * dz, out, t, dt, steps, done, cap, ledger);
     return launch_check(ctx, "diag_finish");
 }
 

@@ -71,57 +71,81 @@ __device__ void merge_partials3_dd(const double* part, int nblocks, double out[6
 
 // accrete! sums over the active-index box [ilo,ihi] x [jlo,jhi] x [klo,khi]:
 // cells with |x - p| < rs and rho > rho_min add rho * rate (and m * rate).
-// The block evaluates the cells' terms in parallel, 1024 at a time, and
-// thread 0 adds them in the reference's (k, j, i) order; a skipped cell adds
-// +0.0, which leaves every sum as skipping it would (an accumulator that
-// starts at +0.0 never becomes -0.0 by adding +0.0 or -0.0).  Thread 0 gets
-// out = {dm, dPx, dPy, dPz}.
+// The block evaluates the cells in parallel, 4 NT at a time (four neighbours
+// per thread), keeps the terms of those that add one in the reference's
+// (k, j, i) order by a prefix sum, and four threads, one per sum, add them in
+// that order.  A cell that adds nothing is left out: the sums are sequential,
+// and only about a third of the box lies in the sphere.  Thread 0 gets
+// out = {dm, dPx, dPy, dPz}.  (4 cells of sink radius: 43 us when one thread
+// added every cell's four terms, zeros included.)
 template <int NT>
 __device__ void sink_sums(const double* U, int nx, int ny, int nz, double dx, double dy, double dz, double x0,
                           double y0, double z0, double px, double py, double pz, double rs, double rate,
                           double rho_min, int ilo, int ihi, int jlo, int jhi, int klo, int khi, double out[4]) {
-    constexpr int CH = 1024;
+    constexpr int CH = 4 * NT;
     __shared__ double term[4][CH];
+    __shared__ int wsum[NT / 32];
+    __shared__ double total4[4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long nI = ihi - ilo + 1, nJ = jhi - jlo + 1, nK = khi - klo + 1;
     const long long total = (nI > 0 && nJ > 0 && nK > 0) ? nI * nJ * nK : 0;
     Geom G(nx, ny, nz);
-    double dm = 0.0, dPx = 0.0, dPy = 0.0, dPz = 0.0;
+    double acc = 0.0;   // threads 0, 32, 64, 96: one sum each
     for (long long base = 0; base < total; base += CH) {
-        for (int e = threadIdx.x; e < CH; e += NT) {
-            long long t = base + e;
-            double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
-            if (t < total) {
-                int a = ilo + (int)(t % nI);
-                long long rr = t / nI;
-                int b = jlo + (int)(rr % nJ), c = klo + (int)(rr / nJ);
-                double xc, yc, zc;
-                f64::cell_xyz(a, b, c, x0, y0, z0, dx, dy, dz, xc, yc, zc);
-                double r = sqrt(sq(xc - px) + sq(yc - py) + sq(zc - pz));
-                if (!(r >= rs)) {
-                    long long o = G.act(a, b, c);
-                    if (!(U[o] <= rho_min)) {
-                        v0 = U[o] * rate;
-                        v1 = U[o + 1] * rate;
-                        v2 = U[o + 2] * rate;
-                        v3 = U[o + 3] * rate;
-                    }
+        double v[4][4];
+        int n = 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const long long t = base + 4 * (long long)threadIdx.x + e;
+            if (t >= total) continue;
+            int a = ilo + (int)(t % nI);
+            long long rr = t / nI;
+            int b = jlo + (int)(rr % nJ), c = klo + (int)(rr / nJ);
+            double xc, yc, zc;
+            f64::cell_xyz(a, b, c, x0, y0, z0, dx, dy, dz, xc, yc, zc);
+            double r = sqrt(sq(xc - px) + sq(yc - py) + sq(zc - pz));
+            if (r >= rs) continue;
+            long long o = G.act(a, b, c);
+            if (U[o] <= rho_min) continue;
+            const double w[4] = {U[o] * rate, U[o + 1] * rate, U[o + 2] * rate, U[o + 3] * rate};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i == n) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) v[i][q] = w[q];
                 }
-            }
-            term[0][e] = v0; term[1][e] = v1; term[2][e] = v2; term[3][e] = v3;
+            ++n;
         }
+        int incl = n;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) wsum[warp] = incl;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            const int m = (int)((total - base) < CH ? (total - base) : CH);
-            for (int e = 0; e < m; ++e) {
-                dm += term[0][e];
-                dPx += term[1][e];
-                dPy += term[2][e];
-                dPz += term[3][e];
+        int at = incl - n, m = 0;
+        for (int w = 0; w < NT / 32; ++w) {
+            if (w < warp) at += wsum[w];
+            m += wsum[w];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i < n) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) term[q][at + i] = v[i][q];
             }
+        __syncthreads();
+        if (lane == 0 && warp < 4) {
+            const double* tq = term[warp];
+#pragma unroll 8
+            for (int e = 0; e < m; ++e) acc += tq[e];
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) { out[0] = dm; out[1] = dPx; out[2] = dPy; out[3] = dPz; }
+    if (lane == 0 && warp < 4) total4[warp] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int q = 0; q < 4; ++q) out[q] = total4[q];
 }
 
 }  // namespace sums
