@@ -283,9 +283,12 @@ __global__ void __launch_bounds__(256) fwd_x_kernel(RhoSrc src, C* W1, const C* 
 }
 
 // Generic strided-line pass over a complex array: lines run along an axis of
-// stride `estride`; a block takes `lines` neighbouring lines (stride 1, the kx
-// axis, length nkx) at a fixed outer index.  Input samples t < n_in are read
-// (the rest are zero); outputs t < n_out are written.
+// stride `estride`; a block takes `lines` neighbouring lines of the list that
+// runs along kx (stride 1, length nkx) and on to the next outer index, so only
+// the last block has idle lanes (nkx = n + 1 is one past a multiple of the
+// block's lines: with blocks that end with kx a ninth of them did almost
+// nothing at n = 128, a fifth at 64).  Input samples t < n_in are read (the
+// rest are zero); outputs t < n_out are written.
 template <class C>
 struct AxisIO {
     const C* in;
@@ -298,18 +301,18 @@ struct AxisIO {
 };
 
 template <class C, int LOGN, bool INV>
-__global__ void __launch_bounds__(256) axis_kernel(AxisIO<C> io, const C* tw, int lines) {
+__global__ void __launch_bounds__(256, sizeof(C) == 8 ? 4 : 2) axis_kernel(AxisIO<C> io, const C* tw, int lines) {
     using Sh = LineShape<LOGN>;
     using R = typename Cx<C>::R;
     constexpr int E = Sh::E, T = Sh::T;
     extern __shared__ __align__(16) unsigned char smraw[];
     C* S = reinterpret_cast<C*>(smraw);
     const int l = threadIdx.x % lines, t = threadIdx.x / lines;
-    const int nbx = (io.nkx + lines - 1) / lines;
-    const long long outer = blockIdx.x / nbx;
-    const int kx = (int)(blockIdx.x % nbx) * lines + l;
-    const bool ok = kx < io.nkx;
-    const C* in = io.in + kx + outer * io.in_ostride;
+    const unsigned line = blockIdx.x * (unsigned)lines + l;   // below 2^31: (n + 1) n of at most 2048
+    const long long outer = line / (unsigned)io.nkx;
+    const int kx = (int)(line % (unsigned)io.nkx);
+    const bool ok = outer < io.nouter;
+    const C* in = io.in + kx + (ok ? outer : 0) * io.in_ostride;
     C v[E];
 #pragma unroll
     for (int k = 0; k < E; ++k) {
@@ -331,7 +334,7 @@ __global__ void __launch_bounds__(256) axis_kernel(AxisIO<C> io, const C* tw, in
 // ky0 = 0, nky = N2 on one GPU; a rank's share of it after the transpose of
 // a z-slab decomposition), z < nz in and out.
 template <class C, int LOGN>
-__global__ void __launch_bounds__(256, 2) z_conv_kernel(C* W2, const typename Cx<C>::R* khat, int nx, int N2, int ny,
+__global__ void __launch_bounds__(256, sizeof(C) == 8 ? 3 : 2) z_conv_kernel(C* W2, const typename Cx<C>::R* khat, int nx, int N2, int ny,
                                                      int nz, int lines, const C* tw, int ky0, int nky) {
     using Sh = LineShape<LOGN>;
     using R = typename Cx<C>::R;
@@ -340,19 +343,19 @@ __global__ void __launch_bounds__(256, 2) z_conv_kernel(C* W2, const typename Cx
     C* S = reinterpret_cast<C*>(smraw);
     const int l = threadIdx.x % lines, t = threadIdx.x / lines;
     const int nkx = nx + 1;
-    const int nbx = (nkx + lines - 1) / lines;
-    const int kyl = blockIdx.x / nbx, ky = ky0 + kyl;
-    const int kx = (int)(blockIdx.x % nbx) * lines + l;
-    const bool ok = kx < nkx;
+    const unsigned at = blockIdx.x * (unsigned)lines + l;   // line of the plane, kx fastest (as axis_kernel)
+    const int kyl = (int)(at / (unsigned)nkx), ky = ky0 + kyl;
+    const int kx = (int)(at % (unsigned)nkx);
+    const bool ok = kyl < nky;
     const long long plane = (long long)nkx * nky;
-    C* line = W2 + kx + (long long)nkx * kyl;
+    C* line = W2 + at;
     C v[E];
 #pragma unroll
     for (int k = 0; k < E; ++k) {   // z = t + k*T < N/2 = nz hold data
         v[k] = (ok && k < E / 2) ? line[plane * (t + k * T)] : Cx<C>::mk(R(0), R(0));
     }
     line_fft<C, LOGN, false>(v, S, ColLayout{lines}, l, t, tw);
-    const int kyf = ky <= ny ? ky : N2 - ky;
+    const int kyf = !ok ? 0 : (ky <= ny ? ky : N2 - ky);
     const R* kh = khat + (ok ? kx : 0) + (long long)nkx * kyf;
 #pragma unroll
     for (int k = 0; k < E; ++k) {
@@ -447,9 +450,9 @@ bsn_status launch_axis(bsn_ctx* ctx, const AxisIO<C>& io, const C* tw) {
     static bool done[64] = {false};
     const size_t sm = G::template col_smem<C>();
     BSN_TRY(smem_optin(ctx, (const void*)axis_kernel<C, LOGN, INV>, sm, done));
-    const long long nbx = (io.nkx + G::col_lines - 1) / G::col_lines;
+    const long long nb = (io.nkx * io.nouter + G::col_lines - 1) / G::col_lines;
     prof_begin(ctx);
-    axis_kernel<C, LOGN, INV><<<(unsigned)(nbx * io.nouter), G::col_lines * LineShape<LOGN>::T, sm, ctx->stream>>>(
+    axis_kernel<C, LOGN, INV><<<(unsigned)nb, G::col_lines * LineShape<LOGN>::T, sm, ctx->stream>>>(
         io, tw, G::col_lines);
     return launch_check(ctx, "fft_y_kernel");
 }
@@ -461,9 +464,9 @@ bsn_status launch_zconv(bsn_ctx* ctx, C* W2, const typename Cx<C>::R* K, const C
     static bool done[64] = {false};
     const size_t sm = G::template col_smem<C>();
     BSN_TRY(smem_optin(ctx, (const void*)z_conv_kernel<C, LOGN>, sm, done));
-    const long long nbx = (nx + 1 + G::col_lines - 1) / G::col_lines;
+    const long long nb = ((long long)(nx + 1) * nky + G::col_lines - 1) / G::col_lines;
     prof_begin(ctx);
-    z_conv_kernel<C, LOGN><<<(unsigned)(nbx * nky), G::col_lines * LineShape<LOGN>::T, sm, ctx->stream>>>(
+    z_conv_kernel<C, LOGN><<<(unsigned)nb, G::col_lines * LineShape<LOGN>::T, sm, ctx->stream>>>(
         W2, K, nx, 2 * ny, ny, nz, G::col_lines, tw, ky0, nky);
     return launch_check(ctx, "z_conv_kernel");
 }
