@@ -23,20 +23,24 @@ OUT = os.path.join(HERE, "bsn", "libbsn.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 BASE = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I" + INCLUDE, "-I" + CSRC]
-FP64_PARITY = {"hydro_f64.cu", "sources_f64.cu", "fmr_f64.cu", "fmr_nlevel.cu", "poisson.cu", "context.cu", "cfl_noalloc.cu",
-               "run_steps.cu", "autotune.cu", "coupled_run.cu", "diagnostics.cu", "relax.cu", "tma_host.cu"}
+FP64_PARITY = {"hydro_f64.cu", "stage_f64_lo.cu", "stage_f64_hi.cu", "sources_f64.cu", "fmr_f64.cu", "fmr_nlevel.cu",
+               "poisson.cu", "context.cu", "cfl_noalloc.cu", "run_steps.cu", "autotune.cu", "coupled_run.cu", "diagnostics.cu", "relax.cu", "tma_host.cu"}
 # the FP32 fast path: approximate division and square root.  The stencil
 # units write every multiply-add out (fmaf, fma.rn.f32x2) and are built
 # without contraction, so their results do not depend on the compiler's
 # contraction choices (each tile variant gives the same bits); the FP32 FFTs
 # keep contraction on.
-FAST = {"stage_fast.cu", "learned.cu", "poisson_f32.cu"}
+FAST = {"stage_fast.cu", "stage_guarded.cu", "learned.cu", "poisson_f32.cu"}
 FAST_FLAGS = ["--ftz=true", "--prec-div=false", "--prec-sqrt=false", "--fmad=true"]
-EXPLICIT_FMA = {"stage_fast.cu", "learned.cu"}
+EXPLICIT_FMA = {"stage_fast.cu", "stage_guarded.cu", "learned.cu"}
+
+
+# minutes each: started first
+SLOW = ("learned.cu", "stage_guarded.cu", "stage_fast.cu", "stage_f64_hi.cu", "stage_f64_lo.cu")
 
 
 def sources():
-    return sorted(f for f in os.listdir(CSRC) if f.endswith(".cu"))
+    return sorted((f for f in os.listdir(CSRC) if f.endswith(".cu")), key=lambda f: (f not in SLOW, f))
 
 
 def _deps_mtime():

@@ -10,6 +10,8 @@
 // by the reference's arithmetic, FP32 by its written-out multiply-adds), so
 // the choice never changes a result.  The choice is stored as a code: the
 // variant index plus kTmaBit when the TMA form won.
+#include <algorithm>
+
 #include "hydro_f64.cuh"
 #include "stage_launch.cuh"
 
@@ -21,11 +23,15 @@ static int variant_count(int prec) {
 static TileVariant variant(int prec, int idx) {
     return prec == PREC_F64 ? f64_variant(idx) : (prec == PREC_F32 ? f32_variant(idx) : learned_variant(idx));
 }
-constexpr int kTmaBit = 256;   // tile-choice code: variant index | kTmaBit when TMA staging is chosen
+// tile-choice code: variant index, | kTmaBit when TMA staging is chosen, or
+// | kListBit when uniform tiles are done apart and the others listed
+constexpr int kTmaBit = 256, kListBit = 512;
 
 // One launch of variant `code & 255`, TMA-staged where the code asks for it
 // (and the grid allows it); ctx->tma_used_last tells whether it was.
-static bsn_status launch_variant(bsn_ctx* ctx, int prec, int code, const f64::StageArgs& A) {
+static bsn_status launch_variant(bsn_ctx* ctx, int prec, int code, const f64::StageArgs& A0) {
+    f64::StageArgs A = A0;
+    if (!(code & kListBit)) A.uni_in = nullptr, A.uni_un = nullptr, A.uni_out = nullptr;
     const int idx = code & (kTmaBit - 1);
     ctx->tma_now = (code & kTmaBit) ? 1 : 0;
     ctx->tma_used_last = 0;
@@ -35,10 +41,11 @@ static bsn_status launch_variant(bsn_ctx* ctx, int prec, int code, const f64::St
     ctx->tma_now = 0;
     return st;
 }
-// the code of a forced variant: TMA wherever the context allows it
-static int forced_code(bsn_ctx* ctx, int prec) {
+// the code of a forced variant: listed where A keeps uniform tiles, else TMA
+// wherever the context allows it
+static int forced_code(bsn_ctx* ctx, int prec, const f64::StageArgs& A) {
     const int v = ctx->forced_tile[prec] >= 0 ? ctx->forced_tile[prec] : 0;
-    return v | (ctx->tma_on ? kTmaBit : 0);
+    return v | (ctx->tma_on ? kTmaBit : 0) | (A.uni_in ? kListBit : 0);
 }
 static bsn_status launch_batch_variant(bsn_ctx* ctx, int prec, int idx, const f64::StageBatch& B) {
     if (prec == PREC_F64) return f64_launch_batch_variant(ctx, idx, B);
@@ -46,10 +53,6 @@ static bsn_status launch_batch_variant(bsn_ctx* ctx, int prec, int idx, const f6
     return learned_launch_batch_variant(ctx, idx, B);
 }
 static bool prec_ok(int p) { return p == PREC_F64 || p == PREC_F32 || p == PREC_LEARNED; }
-// Drivers whose stages run in batched launches over several grids: the batch
-// kernel has no TMA form, so their choices are timed with the plain loader only
-// (a TMA variant timed alone can win and then run plain, and slower, in the batch).
-static bool batched_class(int c) { return c == TUNE_FMR || c == TUNE_FMR_N || c == TUNE_NESTED; }
 static std::tuple<int, int, int, int, int> tile_key(int prec, const f64::StageArgs& A) {
     return std::make_tuple(prec, A.tune_class, A.nx, A.ny, A.nz);
 }
@@ -63,21 +66,89 @@ int tile_code(bsn_ctx* ctx, int prec, const f64::StageArgs& A) {
     return it == ctx->tile_choice.end() ? -1 : it->second;
 }
 
-bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, double* scratch) {
-    if (prec == PREC_LEARNED) {   // the split learned stage's block list, allocated before any capture
-        bsn_status st;
-        slot(ctx, SLOT_SPLIT, learned_split_bytes(probe.nx, probe.ny, probe.nz), &st);
+// One CTA per tile: 1 where all of its active cells hold the same words.
+__global__ void uniform_tiles_kernel(const double* U, int nx, int ny, int nz, int tx, int ty, int tz,
+                                     unsigned char* out) {
+    const Geom G(nx, ny, nz);
+    const int a0 = blockIdx.x * tx, b0 = blockIdx.y * ty, c0 = blockIdx.z * tz;
+    const int row = 5 * min(tx, nx - a0), rows = min(ty, ny - b0), planes = min(tz, nz - c0);
+    __shared__ double first[5];
+    if (threadIdx.x < 5) first[threadIdx.x] = U[G.act(a0, b0, c0) + threadIdx.x];
+    __syncthreads();
+    bool mixed = false;
+    for (int e = threadIdx.x; e < row * rows * planes; e += blockDim.x) {
+        const int w = e % row, r = e / row;
+        const double v = U[G.act(a0, b0 + r % rows, c0 + r / rows) + w];
+        mixed |= __double_as_longlong(v) != __double_as_longlong(first[w % 5]);
+    }
+    const int any = __syncthreads_or(mixed);
+    if (threadIdx.x == 0)
+        out[blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z)] = !any;
+}
+
+static bsn_status find_uniform(bsn_ctx* ctx, const TileVariant& v, const f64::StageArgs& base, const double* U,
+                               unsigned char* f) {
+    const dim3 grid((base.nx + v.tx - 1) / v.tx, (base.ny + v.ty - 1) / v.ty, (base.nz + v.tz - 1) / v.tz);
+    prof_begin(ctx);
+    uniform_tiles_kernel<<<grid, 256, 0, ctx->stream>>>(U, base.nx, base.ny, base.nz, v.tx, v.ty, v.tz, f);
+    return launch_check(ctx, "uniform_tiles_kernel");
+}
+
+// Kept for uniform grids of 2^18 cells (64^3) and more with no sources: below
+// that the extra launch costs what it saves (24^3: 3 us of a 150 us step).
+static bool uniform_tiles_apply(const f64::StageArgs& b) {
+    if (b.mode != 0 || b.Gh || b.ledger || b.use_reg || b.use_bnd || b.F[0] || b.F[1] || b.F[2]) return false;
+    if (b.use_bh | b.use_sg | b.use_sink | b.use_rot | b.use_damp) return false;
+    return (long long)b.nx * b.ny * b.nz >= (1LL << 18);
+}
+
+bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int prec, const f64::StageArgs& base, UniformTiles& t) {
+    t.on = uniform_tiles_apply(base);
+    bsn_status st;
+    if (t.on) {
+        size_t tiles = 0;
+        for (int v = 0; v < variant_count(prec); ++v) {
+            const TileVariant q = variant(prec, v);
+            tiles = std::max(tiles, (size_t)((base.nx + q.tx - 1) / q.tx) * ((base.ny + q.ty - 1) / q.ty) *
+                                        ((base.nz + q.tz - 1) / q.tz));
+        }
+        tiles = (tiles + 255) / 256 * 256;
+        unsigned char* f = (unsigned char*)slot(ctx, SLOT_UNIFORM, 256 + (3 + sizeof(int)) * tiles, &st);
+        BSN_TRY(st);
+        t.count = (unsigned int*)f;
+        t.list = (int*)(f + 256);
+        for (int i = 0; i < 3; ++i) t.f[i] = f + 256 + (sizeof(int) + i) * tiles;
+    }
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(ctx->stream, &cs);
+    if (cs != cudaStreamCaptureStatusNone) {   // no timing during a capture: an earlier choice, or none
+        const int code = tile_code(ctx, prec, base);
+        t.on = t.on && code >= 0 && (code & kListBit);
+        return BSN_OK;
+    }
+    f64::StageArgs p = base;
+    t.set(p, 0);
+    double* scratch = nullptr;
+    if (ctx->forced_tile[prec] < 0 && (tile_code(ctx, prec, base) < 0 || base.tune_class == ctx->retime_class)) {
+        scratch = (double*)slot(ctx, SLOT_UN, sizeof(double) * (size_t)Geom(base.nx, base.ny, base.nz).nelem(), &st);
         BSN_TRY(st);
     }
-    const auto key = tile_key(prec, probe);
-    if (ctx->tile_choice.count(key) && (probe.tune_class != ctx->retime_class || ctx->retimed.count(key)))
-        return BSN_OK;
-    if (probe.tune_class == ctx->retime_class) ctx->retimed.insert(key);
-    int nv = variant_count(prec);
-    if (ctx->forced_tile[prec] >= 0) {
-        record(ctx, prec, probe, forced_code(ctx, prec));
-        return BSN_OK;
-    }
+    BSN_TRY(stage_autotune(ctx, prec, p, scratch));
+    t.on = t.on && (tile_code(ctx, prec, base) & kListBit);
+    return BSN_OK;
+}
+
+bsn_status uniform_tiles_find(bsn_ctx* ctx, int prec, const f64::StageArgs& base, const double* U,
+                              const UniformTiles& t) {
+    if (!t.on) return BSN_OK;
+    const int code = tile_code(ctx, prec, base);
+    const TileVariant v = variant(prec, (code >= 0 ? code : forced_code(ctx, prec, base)) & (kTmaBit - 1));
+    BSN_CUDA(ctx, cudaMemsetAsync(t.count, 0, 6 * sizeof(unsigned int), ctx->stream));
+    return find_uniform(ctx, v, base, U, t.f[0]);
+}
+
+// stage-1 work of a probe, writing to scratch and recording nothing
+static f64::StageArgs probe_args(const f64::StageArgs& probe, double* scratch) {
     f64::StageArgs a = probe;
     a.Un = probe.Uin;
     a.Uout = scratch;
@@ -92,6 +163,84 @@ bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, d
     a.dt_dev = nullptr;
     a.done_dev = nullptr;
     a.ledger = nullptr;
+    return a;
+}
+
+// The drivers whose stages run over several grids at once: one choice for all
+// of them, timed as they run, in one launch over every level.  (Timed level by
+// level, levels of one size share the first one's choice: three 128^3 levels
+// of the binary star took the coarse level's 8x8x8, 16.9 ms per step, where
+// 16x16x8 of 512 threads takes 14.9.)
+bsn_status stage_autotune_batch(bsn_ctx* ctx, int prec, const f64::StageArgs* probes, double* const* scratch, int n) {
+    if (n < 1 || n > f64::MAXLEV) return set_err(ctx, BSN_ERR_ARG, "batch of %d levels", n);
+    bool known = true;
+    for (int l = 0; l < n; ++l) {
+        const auto key = tile_key(prec, probes[l]);
+        known = known && ctx->tile_choice.count(key) &&
+                (probes[l].tune_class != ctx->retime_class || ctx->retimed.count(key));
+    }
+    if (known) return BSN_OK;
+    bsn_status st;
+    unsigned int* queue = (unsigned int*)slot(ctx, SLOT_RED, 64, &st);   // counter, then 4 doubles
+    BSN_TRY(st);
+    f64::StageBatch B;
+    B.nlev = n;
+    B.queue = queue;
+    for (int l = 0; l < n; ++l) {
+        if (prec == PREC_LEARNED) {   // the split learned stage's block list, allocated before any capture
+            slot(ctx, SLOT_SPLIT, learned_split_bytes(probes[l].nx, probes[l].ny, probes[l].nz), &st);
+            BSN_TRY(st);
+        }
+        if (probes[l].tune_class == ctx->retime_class) ctx->retimed.insert(tile_key(prec, probes[l]));
+        B.lv[l] = probe_args(probes[l], scratch[l]);
+        if (probes[l].ledger) B.lv[l].ledger = (double*)queue + 1;   // the ledger's kernels, into spare words
+    }
+    int best = 0;
+    if (ctx->forced_tile[prec] >= 0) {
+        best = forced_code(ctx, prec, B.lv[0]);
+    } else {
+        cudaEvent_t e0, e1;
+        BSN_CUDA(ctx, cudaEventCreate(&e0));
+        BSN_CUDA(ctx, cudaEventCreate(&e1));
+        float best_ms = 1e30f;
+        const bool prof = ctx->profiling;
+        ctx->profiling = false;
+        for (int v = 0; v < variant_count(prec) && st == BSN_OK; ++v)
+            for (int r = 0; r < 3 && st == BSN_OK; ++r) {   // the first a warm-up
+                cudaMemsetAsync(queue, 0, sizeof(unsigned int), ctx->stream);
+                cudaEventRecord(e0, ctx->stream);
+                st = launch_batch_variant(ctx, prec, v, B);
+                cudaEventRecord(e1, ctx->stream);
+                if (st == BSN_OK) st = cuda_check(ctx, cudaEventSynchronize(e1), "cudaEventSynchronize(autotune)");
+                float t = 0.f;
+                cudaEventElapsedTime(&t, e0, e1);
+                if (r > 0 && t < best_ms) { best_ms = t; best = v; }
+            }
+        ctx->profiling = prof;
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        BSN_TRY(st);
+    }
+    for (int l = 0; l < n; ++l) record(ctx, prec, probes[l], best);
+    return BSN_OK;
+}
+
+bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, double* scratch) {
+    if (prec == PREC_LEARNED) {   // the split learned stage's block list, allocated before any capture
+        bsn_status st;
+        slot(ctx, SLOT_SPLIT, learned_split_bytes(probe.nx, probe.ny, probe.nz), &st);
+        BSN_TRY(st);
+    }
+    const auto key = tile_key(prec, probe);
+    if (ctx->tile_choice.count(key) && (probe.tune_class != ctx->retime_class || ctx->retimed.count(key)))
+        return BSN_OK;
+    if (probe.tune_class == ctx->retime_class) ctx->retimed.insert(key);
+    int nv = variant_count(prec);
+    if (ctx->forced_tile[prec] >= 0) {
+        record(ctx, prec, probe, forced_code(ctx, prec, probe));
+        return BSN_OK;
+    }
+    const f64::StageArgs a = probe_args(probe, scratch);
     cudaEvent_t e0, e1;
     BSN_CUDA(ctx, cudaEventCreate(&e0));
     BSN_CUDA(ctx, cudaEventCreate(&e1));
@@ -100,23 +249,35 @@ bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, d
     bool prof = ctx->profiling;
     ctx->profiling = false;
     bsn_status st = BSN_OK;
+    auto timed = [&](auto&& f) -> float {
+        cudaEventRecord(e0, ctx->stream);
+        st = f();
+        cudaEventRecord(e1, ctx->stream);
+        st = st != BSN_OK ? st : cuda_check(ctx, cudaEventSynchronize(e1), "cudaEventSynchronize(autotune)");
+        float t = 0.f;
+        cudaEventElapsedTime(&t, e0, e1);
+        return t;
+    };
+    // one code; extra: time per stage it costs besides its launches.  False:
+    // failed (st), or the grid does not allow this staging
+    auto try_code = [&](int code, float extra) -> bool {
+        float ms = 1e30f;
+        for (int r = 0; r < 3 && st == BSN_OK; ++r) {   // the first a warm-up (sets smem attributes)
+            if (code & kListBit) cudaMemsetAsync(a.list_count, 0, 2 * sizeof(unsigned int), ctx->stream);
+            const float t = timed([&] { return launch_variant(ctx, prec, code, a); });
+            if ((code & kTmaBit) && !ctx->tma_used_last) return false;
+            if (r > 0) ms = t < ms ? t : ms;
+        }
+        if (ms + extra < best_ms) { best_ms = ms + extra; best = code; }
+        return st == BSN_OK;
+    };
     for (int v = 0; v < nv && st == BSN_OK; ++v) {
-        for (int tma = 0; tma < (ctx->tma_on && !batched_class(probe.tune_class) ? 2 : 1) && st == BSN_OK; ++tma) {
-            const int code = v | (tma ? kTmaBit : 0);
-            st = launch_variant(ctx, prec, code, a);   // warm-up (sets smem attributes)
-            if (st != BSN_OK) break;
-            if (tma && !ctx->tma_used_last) break;      // the grid does not allow TMA staging of this tile
-            float ms = 1e30f;
-            for (int r = 0; r < 2 && st == BSN_OK; ++r) {
-                cudaEventRecord(e0, ctx->stream);
-                st = launch_variant(ctx, prec, code, a);
-                cudaEventRecord(e1, ctx->stream);
-                st = st != BSN_OK ? st : cuda_check(ctx, cudaEventSynchronize(e1), "cudaEventSynchronize(autotune)");
-                float t = 0.f;
-                cudaEventElapsedTime(&t, e0, e1);
-                ms = t < ms ? t : ms;
-            }
-            if (ms < best_ms) { best_ms = ms; best = code; }
+        if (try_code(v, 0.f) && ctx->tma_on) try_code(v | kTmaBit, 0.f);
+        if (st == BSN_OK && a.uni_in) {   // single steps find the uniform tiles anew for their three stages
+            const float find = timed([&] {
+                return find_uniform(ctx, variant(prec, v), a, a.Uin, const_cast<unsigned char*>(a.uni_in));
+            });
+            if (st == BSN_OK) try_code(v | kListBit, probe.tune_class == TUNE_GENERIC ? find / 3.f : 0.f);
         }
     }
     ctx->profiling = prof;
@@ -147,7 +308,7 @@ bsn_status stage_launch(bsn_ctx* ctx, int prec, const f64::StageArgs& A) {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         cudaStreamIsCapturing(ctx->stream, &cs);
         if (ctx->forced_tile[prec] >= 0 || cs != cudaStreamCaptureStatusNone)
-            return launch_variant(ctx, prec, forced_code(ctx, prec), A);
+            return launch_variant(ctx, prec, forced_code(ctx, prec, A), A);
         Geom G(A.nx, A.ny, A.nz);
         bsn_status st;
         double* scratch = (double*)slot(ctx, SLOT_UN, sizeof(double) * (size_t)G.nelem(), &st);

@@ -3,7 +3,6 @@
 // Compiled with -fmad=false: bit-identical to the reference's CPU arithmetic.
 #include "hydro_f64.cuh"
 #include "stage_launch.cuh"
-#include "stage_tile.cuh"
 
 namespace bsn {
 namespace f64 {
@@ -206,41 +205,19 @@ void stage_args_init(StageArgs& A, int nx, int ny, int nz, double dx, double dy,
 
 // FP64 tile variants of the fused stage kernel (bitwise identical results:
 // every interface and every cell is computed by the same arithmetic whatever
-// the tiling).  MINB keeps two 256-thread CTAs (or the equivalent) per SM.
+// the tiling); their kernels are stage_f64_lo.cu's and stage_f64_hi.cu's.
+// MINB keeps two 256-thread CTAs (or the equivalent) per SM.
 namespace {
 const TileVariant kF64Variants[] = {{8, 8, 8, 256, 2}, {8, 8, 4, 128, 4}, {16, 8, 4, 256, 2}, {16, 8, 8, 512, 1}};
-
-template <int TX, int TY, int TZ, int NT, int MINB>
-bsn_status launch_f64(bsn_ctx* ctx, const StageArgs& A) {
-    bool tma_used = false;
-    BSN_TRY((tile::launch_tma<tile::F64Physics, TX, TY, TZ, NT, MINB>(ctx, A, "stage_kernel_tma", &tma_used)));
-    if (tma_used) return BSN_OK;
-    return tile::launch_plain<tile::F64Physics, TX, TY, TZ, NT, MINB>(
-        ctx, A, tile::smem_bytes<tile::F64Physics, TX, TY, TZ>(), "stage_kernel");
-}
 }  // namespace
 
 int f64_variant_count() { return (int)(sizeof(kF64Variants) / sizeof(kF64Variants[0])); }
 TileVariant f64_variant(int idx) { return kF64Variants[idx]; }
 bsn_status f64_launch_variant(bsn_ctx* ctx, int idx, const StageArgs& A) {
-    switch (idx) {
-        case 0: return launch_f64<8, 8, 8, 256, 2>(ctx, A);
-        case 1: return launch_f64<8, 8, 4, 128, 4>(ctx, A);
-        case 2: return launch_f64<16, 8, 4, 256, 2>(ctx, A);
-        case 3: return launch_f64<16, 8, 8, 512, 1>(ctx, A);
-        default: return set_err(ctx, BSN_ERR_ARG, "no FP64 tile variant %d", idx);
-    }
+    return idx < 2 ? f64_launch_variant_lo(ctx, idx, A) : f64_launch_variant_hi(ctx, idx, A);
 }
-
 bsn_status f64_launch_batch_variant(bsn_ctx* ctx, int idx, const StageBatch& B) {
-    using P = tile::F64Physics;
-    switch (idx) {
-        case 0: return tile::launch_batch<P, 8, 8, 8, 256, 2>(ctx, B, tile::smem_bytes<P, 8, 8, 8>(), "stage_kernel_batch");
-        case 1: return tile::launch_batch<P, 8, 8, 4, 128, 4>(ctx, B, tile::smem_bytes<P, 8, 8, 4>(), "stage_kernel_batch");
-        case 2: return tile::launch_batch<P, 16, 8, 4, 256, 2>(ctx, B, tile::smem_bytes<P, 16, 8, 4>(), "stage_kernel_batch");
-        case 3: return tile::launch_batch<P, 16, 8, 8, 512, 1>(ctx, B, tile::smem_bytes<P, 16, 8, 8>(), "stage_kernel_batch");
-        default: return set_err(ctx, BSN_ERR_ARG, "no FP64 tile variant %d", idx);
-    }
+    return idx < 2 ? f64_launch_batch_variant_lo(ctx, idx, B) : f64_launch_batch_variant_hi(ctx, idx, B);
 }
 
 bsn_status f64_launch_stage(bsn_ctx* ctx, const StageArgs& A) { return stage_launch(ctx, PREC_F64, A); }
@@ -262,9 +239,17 @@ bsn_status f64_rk3(bsn_ctx* ctx, StageArgs base, double* U, double dt, const dou
     double* B = (double*)slot(ctx, SLOT_B, bytes, &st); BSN_TRY(st);
     double* in[3] = {U, A, B};
     double* out[3] = {A, B, U};
+    UniformTiles uni;
+    if (!phi_per_stage) {
+        base.Uin = U;
+        base.Un = U;
+        BSN_TRY(uniform_tiles_prepare(ctx, PREC_F64, base, uni));
+        BSN_TRY(uniform_tiles_find(ctx, PREC_F64, base, U, uni));
+    }
     for (int s = 0; s < 3; ++s) {
         StageArgs a = base;
         a.Uin = in[s]; a.Un = U; a.Uout = out[s]; a.mode = 0;
+        uni.set(a, s);
         set_stage(a, s + 1, dt);
         if (phi_per_stage) { a.phi = phi_per_stage[s]; a.use_sg = phi_per_stage[s] != nullptr; }
         a.cfl_max = (s == 2) ? cfl_max : nullptr;

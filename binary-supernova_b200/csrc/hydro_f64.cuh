@@ -47,6 +47,22 @@ bsn_status cfl_from_device(bsn_ctx* ctx, const unsigned long long* red, double c
 bsn_status graph_replay(bsn_ctx* ctx, cudaGraphExec_t exec, int kernels, int n_steps, bool until_done,
                         const int* done_dev, cudaEvent_t ev[2], volatile int* hflag);
 
+// Steps that a call on buffers without a captured graph takes as plain
+// launches: capturing and instantiating a graph costs about 180 us of host
+// time, while the launches of a step (12 to 45, some 2 us each) go on ahead of
+// the GPU.  64^3 coupled loop, 2 steps on new buffers: 1.96 ms with a graph
+// captured for them, 1.79 ms replaying one that is there.
+constexpr int kDirectSteps = 4;
+template <class F>
+bsn_status launch_steps(bsn_ctx* ctx, F&& body, int n_steps) {
+    const bool prof = ctx->profiling;   // as the graphs, outside the per-kernel records
+    ctx->profiling = false;
+    bsn_status st = BSN_OK;
+    for (int i = 0; i < n_steps && st == BSN_OK; ++i) st = body();
+    ctx->profiling = prof;
+    return st;
+}
+
 // r_sink / t_sink of src/BinarySupernova.jl:159-171 (host FP64).
 inline double bh_r_sink(const bsn_bh& b) {
     double v = 6.0 * b.mass / (b.c_code * b.c_code);

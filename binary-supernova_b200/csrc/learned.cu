@@ -458,7 +458,7 @@ struct State {
 namespace tile {
 
 struct F32Learned {
-    static constexpr bool kStiffFallback = false;   // the warp path reconstructs all faces in FP32
+    static constexpr bool kDeferred = false;   // the warp path reconstructs all faces in FP32
     using real = float;
     static constexpr bool kCenterFromSmem = false;
     static constexpr bool kWarpFaces = true;
@@ -497,32 +497,10 @@ struct F32Learned {
         uint4* dst = (uint4*)psm;                 // policy_smem: 16-byte aligned
         for (int i = threadIdx.x; i < 2 * learned::PK_BYTES / 16; i += nt) dst[i] = src[i];
     }
-    // P clamp, face energy and HLLC of one interface from its reconstructed
-    // (rho, m, P) on both sides (the FP32 path's arithmetic), with the sweep
-    // direction at run time (the warp path below is one function for all
-    // three sweeps)
-    __device__ static void finish_rt(const float (&c)[6][6], const Consts& k, const float (&L)[5], const float (&Rv)[5],
-                                     float (&F)[5], int D) {
-        float PmaxL = fmaxf(fmaxf(fmaxf(fmaxf(c[0][5], c[1][5]), c[2][5]), c[3][5]), c[4][5]);
-        float PmaxR = fmaxf(fmaxf(fmaxf(fmaxf(c[1][5], c[2][5]), c[3][5]), c[4][5]), c[5][5]);
-        float PL = fminf(fmaxf(L[4], 0.0f), PmaxL);
-        float PR = fminf(fmaxf(Rv[4], 0.0f), PmaxR);
-        float EL = f32::EL_from_P(PL, L[0], L[1], L[2], L[3], k.inv_gm1);
-        float ER = f32::EL_from_P(PR, Rv[0], Rv[1], Rv[2], Rv[3], k.inv_gm1);
-        // (normal, t1, t2) = (x, y, z), (y, x, z), (z, x, y)
-        const float nL = D == 0 ? L[1] : (D == 1 ? L[2] : L[3]);
-        const float aL = D == 0 ? L[2] : L[1];
-        const float bL = D == 2 ? L[2] : L[3];
-        const float nR = D == 0 ? Rv[1] : (D == 1 ? Rv[2] : Rv[3]);
-        const float aR = D == 0 ? Rv[2] : Rv[1];
-        const float bR = D == 2 ? Rv[2] : Rv[3];
-        float Fr[5];
-        f32::hllc_normal(L[0], nL, aL, bL, EL, Rv[0], nR, aR, bR, ER, k.g, k.gm1, k.gg, Fr);
-        F[0] = Fr[0];
-        F[1] = D == 0 ? Fr[1] : Fr[2];
-        F[2] = D == 0 ? Fr[2] : (D == 1 ? Fr[1] : Fr[3]);
-        F[3] = D == 2 ? Fr[1] : Fr[3];
-        F[4] = Fr[4];
+    // the FP32 path's end of a face
+    __device__ __forceinline__ static void finish(const float (&c)[6][6], const Consts& k, const float (&L)[5],
+                                                  const float (&Rv)[5], float (&F)[5], int D) {
+        f32::finish_face(c, L, Rv, k.g, k.gm1, k.inv_gm1, k.gg, D, F);
     }
     // One interface per lane; every lane of the warp calls this (valid or not).
     // c[cell][col]: cols 0-3 rho, m_x, m_y, m_z, col 4 E, col 5 P; the
@@ -540,26 +518,17 @@ struct F32Learned {
     // (prefix sum of the lanes' counts), one side at a time, so the tensor
     // cores run ceil(rows / 16) tiles and none when the warp's stencils are
     // all quiescent or shocked.
-    template <int D>
-    __device__ static void warp_flux(const float (&c)[6][6], bool valid, const Consts& k, float F[5],
-                                     unsigned char* psm, int warp, bool quiet) {
-        float Fo[5];
-        warp_flux_rt(c, valid, k, Fo, psm, warp, quiet, D);
-#pragma unroll
-        for (int q = 0; q < 5; ++q) F[q] = Fo[q];
-    }
-    // Inlined into each sweep with D a compile-time constant: an out-of-line
+    // Inlined into each sweep (D is a constant after inlining): an out-of-line
     // copy shrinks the kernel's code but passes the stencil and the caller's
     // live registers through local memory on every call, which costs more
     // than it saves where most sweeps are non-uniform (inside a star).
-    __device__ __forceinline__ static void warp_flux_rt(const float (&c)[6][6], bool valid, const Consts& k,
-                                                        float (&F)[5], unsigned char* psm, int warp, bool quiet,
-                                                        int D) {
+    __device__ __forceinline__ static void warp_flux(const float (&c)[6][6], bool valid, const Consts& k, float (&F)[5],
+                                                     unsigned char* psm, int warp, bool quiet, int D) {
         const int lane = threadIdx.x & 31;
         uint32_t* R = (uint32_t*)(psm + 2 * learned::PK_BYTES + warp * 160 * 16);
         float* logit = (float*)R;
         const float t13 = 1.0f / 3.0f, m76 = -7.0f / 6.0f, e116 = 11.0f / 6.0f, m16 = -1.0f / 6.0f,
-                    f56 = 5.0f / 6.0f, k1312 = 13.0f / 12.0f;
+                    f56 = 5.0f / 6.0f;
         float L[5], Rv[5];
         unsigned need[2] = {0u, 0u};
         // the smoothness test of field q from its stencil and indicators
@@ -608,29 +577,14 @@ struct F32Learned {
             const int q = 4, col = 5;
             float c0 = c[0][col], c1 = c[1][col], c2 = c[2][col], c3 = c[3][col], c4 = c[4][col], c5 = c[5][col];
             if (!valid) c0 = c1 = c2 = c3 = c4 = c5 = 0.f;
-            // f32::weno5_lr's operations, keeping the indicators for the test
-            float qA = fmaf(e116, c2, fmaf(m76, c1, t13 * c0));
-            float qB = fmaf(t13, c3, fmaf(f56, c2, m16 * c1));
-            float qC = fmaf(m16, c4, fmaf(f56, c3, t13 * c2));
-            float qD = fmaf(t13, c5, fmaf(m76, c4, e116 * c3));
-            float s0 = fmaf(-2.0f, c1, c0) + c2, s1 = fmaf(-2.0f, c2, c1) + c3, s2 = fmaf(-2.0f, c3, c2) + c4,
-                  s3 = fmaf(-2.0f, c4, c3) + c5;
-            float a = fmaf(3.0f, c2, fmaf(-4.0f, c1, c0)), b = c1 - c3, cc = fmaf(-4.0f, c3, 3.0f * c2) + c4,
-                  d = fmaf(3.0f, c4, fmaf(-4.0f, c3, c2)), e = fmaf(-4.0f, c4, 3.0f * c3) + c5;
-            float bA = fmaf(k1312 * s0, s0, 0.25f * a * a);
-            float bB = fmaf(k1312 * s1, s1, 0.25f * b * b);
-            float x2 = k1312 * s2 * s2;
-            float bC = fmaf(0.25f * cc, cc, x2);
-            float bD = fmaf(0.25f * d, d, x2);
-            float bE = fmaf(k1312 * s3, s3, 0.25f * e * e);
-            L[q] = f32::wz(bA, bB, bC, 0.1f, 0.6f, 0.3f, qA, qB, qC);
-            Rv[q] = f32::wz(bB, bD, bE, 0.3f, 0.6f, 0.1f, qB, qC, qD);
+            float bA, bB, bC, bD, bE;
+            f32::weno5_lr(c0, c1, c2, c3, c4, c5, L[q], Rv[q], bA, bB, bC, bD, bE);
             if (!quiet) test(q, c0, c1, c2, c3, c4, c5, bA, bB, bC, bD, bE);
         }
-        if (quiet) return finish_rt(c, k, L, Rv, F, D);
+        if (quiet) return finish(c, k, L, Rv, F, D);
         // both sides' row counts in one prefix sum (8 bits each: at most 160 rows a side)
         const int packed = __popc(need[0]) | (__popc(need[1]) << 8);
-        if (!__any_sync(0xffffffffu, packed != 0)) return finish_rt(c, k, L, Rv, F, D);   // warp-uniform
+        if (!__any_sync(0xffffffffu, packed != 0)) return finish(c, k, L, Rv, F, D);   // warp-uniform
         int incl = packed;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -693,12 +647,12 @@ struct F32Learned {
             }
             __syncwarp();
         }
-        finish_rt(c, k, L, Rv, F, D);
+        finish(c, k, L, Rv, F, D);
     }
-    template <int D>
     // uniform sweeps (kQuiescentSkip): no network row can occur, plain FP32 WENO5-Z + HLLC
-    __device__ static void flux(const float (&c)[6][6], const Consts& k, float F[5]) {
-        f32::interface_flux<D>(c, k.g, k.gm1, k.inv_gm1, k.gg, F);
+    __device__ __forceinline__ static bool flux(const float (&c)[6][6], const Consts& k, int D, float F[5]) {
+        f32::interface_flux(c, k.g, k.gm1, k.inv_gm1, k.gg, D, F);
+        return false;
     }
 };
 
@@ -733,27 +687,9 @@ bsn_status launch_learned_whole(bsn_ctx* ctx, const f64::StageArgs& A) {
 template <int TX, int TY, int TZ, int NT, int MINB>
 bsn_status launch_learned(bsn_ctx* ctx, const f64::StageArgs& A0) {
     if (!A0.learned_split) return launch_learned_whole<TX, TY, TZ, NT, MINB>(ctx, A0);
-    auto fs = tile::stage_kernel<tile::F32Screen, TX, TY, TZ, NT, MINB>;
-    auto fl = tile::stage_kernel_list<tile::F32Learned, TX, TY, TZ, NT, MINB>;
     constexpr int smem_s = tile::smem_bytes<tile::F32Screen, TX, TY, TZ>();
     constexpr int smem_l = tile::smem_bytes<tile::F32Learned, TX, TY, TZ>() + tile::F32Learned::kExtraSmem(NT) + 16;
     static_assert(smem_s <= 232448 && smem_l <= 232448, "tile's shared memory exceeds the per-CTA limit");
-    static int occ[64] = {0}, sms[64] = {0};
-    int dev = ctx->device & 63;
-    if (!occ[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(fs, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_s);
-        if (e != cudaSuccess) return cuda_check(ctx, e, "cudaFuncSetAttribute(stage_kernel_learned_screen)");
-        e = cudaFuncSetAttribute(fl, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_l);
-        if (e != cudaSuccess) return cuda_check(ctx, e, "cudaFuncSetAttribute(stage_kernel_learned)");
-        int o = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fl, NT, smem_l);
-        if (e != cudaSuccess) return cuda_check(ctx, e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-        e = cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, ctx->device);
-        if (e != cudaSuccess) return cuda_check(ctx, e, "cudaDeviceGetAttribute");
-        occ[dev] = o < 1 ? 1 : o;
-    }
-    dim3 grid((A0.nx + TX - 1) / TX, (A0.ny + TY - 1) / TY, (A0.nz + TZ - 1) / TZ);
-    const long long nblk = (long long)grid.x * grid.y * grid.z;
     bsn_status st;
     // sized for every variant before any graph capture (stage_autotune), so this never allocates while capturing
     unsigned int* cnt = (unsigned int*)slot(ctx, SLOT_SPLIT, learned_split_bytes(A0.nx, A0.ny, A0.nz), &st);
@@ -763,13 +699,16 @@ bsn_status launch_learned(bsn_ctx* ctx, const f64::StageArgs& A0) {
     A.split_list = (int*)(cnt + 4);
     BSN_CUDA(ctx, cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned int), ctx->stream));   // list count, queue counter
     // the screening launch stages with the plain loader (its TMA form is not used)
-    prof_begin(ctx);
-    fs<<<grid, NT, smem_s, ctx->stream>>>(A);
-    BSN_TRY(launch_check(ctx, "stage_kernel_learned_screen"));
-    const long long pgrid = std::min<long long>(nblk, (long long)occ[dev] * sms[dev]);
-    prof_begin(ctx);
-    fl<<<(unsigned)pgrid, NT, smem_l, ctx->stream>>>(A);
-    return launch_check(ctx, "stage_kernel_learned");
+    if (A.uni_in) {
+        BSN_TRY(tile::launch_uniform<tile::F32Screen>(ctx, A, TX, TY, TZ));
+        BSN_TRY((tile::launch_list<tile::F32Screen, TX, TY, TZ, NT, MINB>(ctx, A, smem_s, "stage_kernel_learned_screen")));
+    } else {
+        BSN_TRY((tile::launch_plain_led<tile::F32Screen, TX, TY, TZ, NT, MINB, false>(ctx, A, smem_s,
+                                                                                     "stage_kernel_learned_screen")));
+    }
+    A.list = A.split_list;
+    A.list_count = A.split_count;
+    return tile::launch_list<tile::F32Learned, TX, TY, TZ, NT, MINB>(ctx, A, smem_l, "stage_kernel_learned");
 }
 }  // namespace
 

@@ -185,13 +185,23 @@ __device__ __forceinline__ void interface_flux(const double (&c)[6][6], double g
     }
 }
 
+// hm2 / r, IEEE-rounded: the kinetic energy of a cell (hm2 = 0.5 m^2).  Gas at
+// rest, the most common cell of an atmosphere, needs no division.
+__device__ __forceinline__ double kinetic(double hm2, double r) {
+    if (abs_hi(r) - hi_pow2(-100) < hi_pow2(116) - hi_pow2(-100) && r > 0.0 && abs_hi(hm2) < hi_pow2(240)) {
+        if (hm2 == 0.0) return 0.0;
+        if (!too_small(hm2, kNumRhoLo)) return quot_pos(hm2, r, recip_rn(r));
+    }
+    return hm2 / r;
+}
+
 // Density/pressure floors (src/gpu_kernels.jl:26-46).  Pfl_gm1 = P_floor/(gamma-1).
 __device__ __forceinline__ void apply_floor(double& r, double& mx, double& my, double& mz, double& E,
                                             double rho_floor, double P_floor, double Pfl_gm1, double gm1) {
     if (r < rho_floor) {
         r = rho_floor; mx = 0.0; my = 0.0; mz = 0.0; E = Pfl_gm1;
     } else {
-        double KE = 0.5 * (sq(mx) + sq(my) + sq(mz)) / r;
+        double KE = kinetic(0.5 * (sq(mx) + sq(my) + sq(mz)), r);
         double P = gm1 * (E - KE);
         if (P < P_floor) E = Pfl_gm1 + KE;
     }
@@ -362,11 +372,11 @@ __device__ __forceinline__ bool EL_from_P_ord(double PL, double rL, double y, do
     return too_small(PL, kNumRhoLo);
 }
 
-// interface_flux for ordinary cells; gg = (g + 1) / (2 g), igm1 = RN(1 / gm1).
-// Returns true where the general interface_flux must be taken instead.
-template <int D>
+// interface_flux along axis D (a constant, or at run time) for ordinary cells;
+// gg = (g + 1) / (2 g), igm1 = RN(1 / gm1).  Returns true where the general
+// interface_flux must be taken instead.
 __device__ __forceinline__ bool interface_flux_ord(const double (&c)[6][6], double g, double gm1, double igm1,
-                                                   double gg, double F[5]) {
+                                                   double gg, int D, double F[5]) {
     double L[5], R[5], PL, PR;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
@@ -382,12 +392,27 @@ __device__ __forceinline__ bool interface_flux_ord(const double (&c)[6][6], doub
     double EL, ER;
     bool bad = EL_from_P_ord(PL, L[0], yL, L[1], L[2], L[3], gm1, igm1, &EL);
     bad |= EL_from_P_ord(PR, R[0], yR, R[1], R[2], R[3], gm1, igm1, &ER);
-    constexpr int n = D + 1, a = D == 0 ? 2 : 1, b = D == 2 ? 2 : 3;   // (normal, t1, t2)
+    // (normal, t1, t2) = (x, y, z), (y, x, z), (z, x, y)
     double Fr[5];
-    bad |= hllc_normal_ord(L[0], yL, L[n], L[a], L[b], EL, R[0], yR, R[n], R[a], R[b], ER, g, gm1, gg, Fr);
-    F[0] = Fr[0]; F[n] = Fr[1]; F[a] = Fr[2]; F[b] = Fr[3]; F[4] = Fr[4];
+    bad |= hllc_normal_ord(L[0], yL, D == 0 ? L[1] : (D == 1 ? L[2] : L[3]), D == 0 ? L[2] : L[1],
+                           D == 2 ? L[2] : L[3], EL, R[0], yR, D == 0 ? R[1] : (D == 1 ? R[2] : R[3]),
+                           D == 0 ? R[2] : R[1], D == 2 ? R[2] : R[3], ER, g, gm1, gg, Fr);
+    F[0] = Fr[0];
+    F[1] = D == 0 ? Fr[1] : Fr[2];
+    F[2] = D == 0 ? Fr[2] : (D == 1 ? Fr[1] : Fr[3]);
+    F[3] = D == 2 ? Fr[1] : Fr[3];
+    F[4] = Fr[4];
     return bad;
 }
+
+// interface_flux along axis D, out of line: the rare faces of interface_flux_ord
+__device__ __noinline__ inline void general_flux(const double (&c)[6][6], double g, double gm1, int D, double F[5]) {
+    if (D == 0) interface_flux<0>(c, g, gm1, F);
+    else if (D == 1) interface_flux<1>(c, g, gm1, F);
+    else interface_flux<2>(c, g, gm1, F);
+}
+// a gamma - 1 that quot can divide pressures by
+__device__ __forceinline__ bool ordinary_gamma(double gm1) { return gm1 >= 0x1p-20 && gm1 < 0x1p20; }
 
 // apply_floor (active cells) and cell_pressure of one cell with one division:
 // both use the cell's kinetic energy.  Returns true when the cell is

@@ -27,46 +27,13 @@ namespace f32 {
 // differences; a denominator above 2^126 would need state values beyond
 // 1e18, far outside what the path represents.
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
-
-__device__ __forceinline__ float wz(float b0, float b1, float b2, float d0, float d1, float d2, float q0, float q1,
-                                    float q2) {
-    const float eps = 1e-36f, cap = 1e18f;
-    float tau = fabsf(b0 - b2);
-    float t0 = fminf(fdiv(tau, eps + b0), cap);
-    float t1 = fminf(fdiv(tau, eps + b1), cap);
-    float t2 = fminf(fdiv(tau, eps + b2), cap);
-    float a0 = d0 * fmaf(t0, t0, 1.0f);
-    float a1 = d1 * fmaf(t1, t1, 1.0f);
-    float a2 = d2 * fmaf(t2, t2, 1.0f);
-    float num = fmaf(a0, q0, fmaf(a1, q1, a2 * q2));
-    return fdiv(num, a0 + a1 + a2);
-}
-
-// Left/right WENO5-Z at the interface between c2 and c3 (src/weno5.jl:25-61).
-__device__ __forceinline__ void weno5_lr(float c0, float c1, float c2, float c3, float c4, float c5, float& L,
-                                         float& R) {
-    const float t13 = 1.0f / 3.0f, m76 = -7.0f / 6.0f, e116 = 11.0f / 6.0f, m16 = -1.0f / 6.0f, f56 = 5.0f / 6.0f;
-    const float k1312 = 13.0f / 12.0f;
-    // the same operations, multiply-adds and order as the two-lane weno5_lr2
-    float qA = fmaf(e116, c2, fmaf(m76, c1, t13 * c0));
-    float qB = fmaf(t13, c3, fmaf(f56, c2, m16 * c1));
-    float qC = fmaf(m16, c4, fmaf(f56, c3, t13 * c2));
-    float qD = fmaf(t13, c5, fmaf(m76, c4, e116 * c3));
-    float s0 = fmaf(-2.0f, c1, c0) + c2, s1 = fmaf(-2.0f, c2, c1) + c3, s2 = fmaf(-2.0f, c3, c2) + c4,
-          s3 = fmaf(-2.0f, c4, c3) + c5;
-    float a = fmaf(3.0f, c2, fmaf(-4.0f, c1, c0));
-    float b = c1 - c3;
-    float c = fmaf(-4.0f, c3, 3.0f * c2) + c4;
-    float d = fmaf(3.0f, c4, fmaf(-4.0f, c3, c2));
-    float e = fmaf(-4.0f, c4, 3.0f * c3) + c5;
-    float bA = fmaf(k1312 * s0, s0, 0.25f * a * a);
-    float bB = fmaf(k1312 * s1, s1, 0.25f * b * b);
-    float x2 = k1312 * s2 * s2;
-    float bC = fmaf(0.25f * c, c, x2);
-    float bD = fmaf(0.25f * d, d, x2);
-    float bE = fmaf(k1312 * s3, s3, 0.25f * e * e);
-    L = wz(bA, bB, bC, 0.1f, 0.6f, 0.3f, qA, qB, qC);
-    R = wz(bB, bD, bE, 0.3f, 0.6f, 0.1f, qB, qC, qD);
+// The reciprocal in it: fdiv(a, b) is a * rcp(b) bit for bit for such b, so
+// quotients by one denominator share it (one of the special-function unit's
+// sixteen lanes per cycle, which a face needs fifty times).
+__device__ __forceinline__ float rcp(float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return y;
 }
 
 // Two FP32 lanes in one 64-bit register pair.  sm_100's packed FP32
@@ -104,24 +71,29 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
     return d;
 }
 
-// wz on two lanes: the same expressions as wz, lane by lane
-__device__ __forceinline__ f2 wz2(f2 b0, f2 b1, f2 b2, float d0, float d1, float d2, f2 q0, f2 q1, f2 q2) {
+// WENO-Z weights and the weighted sum (src/weno5.jl:14-21, 40, 60) on two
+// lanes; (r0x, r0y) ...: rcp of eps + b0 ... per lane
+struct r2 { float x, y; };
+__device__ __forceinline__ r2 rcp_eps(f2 b) {
+    f2 e = sp2(1e-36f) + b;
+    r2 r;
+    up2(e, r.x, r.y);
+    r.x = rcp(r.x);
+    r.y = rcp(r.y);
+    return r;
+}
+__device__ __forceinline__ f2 wz2(f2 b0, f2 b2, r2 y0, r2 y1, r2 y2, f2 d0, f2 d1, f2 d2, f2 q0, f2 q1, f2 q2) {
     const float cap = 1e18f;
-    const f2 eps = sp2(1e-36f), one = sp2(1.0f);
-    f2 dt = b0 - b2;
-    f2 e0 = eps + b0, e1 = eps + b1, e2 = eps + b2;
-    float x, y, ex, ey;
-    up2(dt, x, y);
+    const f2 one = sp2(1.0f);
+    float x, y;
+    up2(b0 - b2, x, y);
     const float taux = fabsf(x), tauy = fabsf(y);
-    up2(e0, ex, ey);
-    f2 t0 = pk2(fminf(fdiv(taux, ex), cap), fminf(fdiv(tauy, ey), cap));
-    up2(e1, ex, ey);
-    f2 t1 = pk2(fminf(fdiv(taux, ex), cap), fminf(fdiv(tauy, ey), cap));
-    up2(e2, ex, ey);
-    f2 t2 = pk2(fminf(fdiv(taux, ex), cap), fminf(fdiv(tauy, ey), cap));
-    f2 a0 = sp2(d0) * fma2(t0, t0, one);
-    f2 a1 = sp2(d1) * fma2(t1, t1, one);
-    f2 a2 = sp2(d2) * fma2(t2, t2, one);
+    f2 t0 = pk2(fminf(taux * y0.x, cap), fminf(tauy * y0.y, cap));
+    f2 t1 = pk2(fminf(taux * y1.x, cap), fminf(tauy * y1.y, cap));
+    f2 t2 = pk2(fminf(taux * y2.x, cap), fminf(tauy * y2.y, cap));
+    f2 a0 = d0 * fma2(t0, t0, one);
+    f2 a1 = d1 * fma2(t1, t1, one);
+    f2 a2 = d2 * fma2(t2, t2, one);
     f2 num = fma2(a0, q0, fma2(a1, q1, a2 * q2));
     f2 den = a0 + a1 + a2;
     float nx, ny, dx, dy;
@@ -155,12 +127,48 @@ __device__ __forceinline__ void weno5_lr2(f2 c0, f2 c1, f2 c2, f2 c3, f2 c4, f2 
     bC = fma2(q4 * c, c, x2);
     bD = fma2(q4 * d, d, x2);
     bE = fma2(k1312 * s3, s3, q4 * e * e);
-    L = wz2(bA, bB, bC, 0.1f, 0.6f, 0.3f, qA, qB, qC);
-    R = wz2(bB, bD, bE, 0.3f, 0.6f, 0.1f, qB, qC, qD);
+    const f2 d1 = sp2(0.1f), d3 = sp2(0.3f), d6 = sp2(0.6f);
+    const r2 yB = rcp_eps(bB);
+    L = wz2(bA, bC, rcp_eps(bA), yB, rcp_eps(bC), d1, d6, d3, qA, qB, qC);
+    R = wz2(bB, bE, yB, rcp_eps(bD), rcp_eps(bE), d3, d6, d1, qB, qC, qD);
 }
 __device__ __forceinline__ void weno5_lr2(f2 c0, f2 c1, f2 c2, f2 c3, f2 c4, f2 c5, f2& L, f2& R) {
     f2 bA, bB, bC, bD, bE;
     weno5_lr2(c0, c1, c2, c3, c4, c5, L, R, bA, bB, bC, bD, bE);
+}
+
+// Left/right WENO5-Z of one field at the interface between c2 and c3
+// (src/weno5.jl:25-61): the same operations, multiply-adds and order as a lane
+// of weno5_lr2, with the two sides as the lanes of the weights.
+__device__ __forceinline__ void weno5_lr(float c0, float c1, float c2, float c3, float c4, float c5, float& L,
+                                         float& R, float& bA, float& bB, float& bC, float& bD, float& bE) {
+    const float t13 = 1.0f / 3.0f, m76 = -7.0f / 6.0f, e116 = 11.0f / 6.0f, m16 = -1.0f / 6.0f, f56 = 5.0f / 6.0f;
+    const float k1312 = 13.0f / 12.0f, eps = 1e-36f;
+    float qA = fmaf(e116, c2, fmaf(m76, c1, t13 * c0));
+    float qB = fmaf(t13, c3, fmaf(f56, c2, m16 * c1));
+    float qC = fmaf(m16, c4, fmaf(f56, c3, t13 * c2));
+    float qD = fmaf(t13, c5, fmaf(m76, c4, e116 * c3));
+    float s0 = fmaf(-2.0f, c1, c0) + c2, s1 = fmaf(-2.0f, c2, c1) + c3, s2 = fmaf(-2.0f, c3, c2) + c4,
+          s3 = fmaf(-2.0f, c4, c3) + c5;
+    float a = fmaf(3.0f, c2, fmaf(-4.0f, c1, c0));
+    float b = c1 - c3;
+    float c = fmaf(-4.0f, c3, 3.0f * c2) + c4;
+    float d = fmaf(3.0f, c4, fmaf(-4.0f, c3, c2));
+    float e = fmaf(-4.0f, c4, 3.0f * c3) + c5;
+    bA = fmaf(k1312 * s0, s0, 0.25f * a * a);
+    bB = fmaf(k1312 * s1, s1, 0.25f * b * b);
+    float x2 = k1312 * s2 * s2;
+    bC = fmaf(0.25f * c, c, x2);
+    bD = fmaf(0.25f * d, d, x2);
+    bE = fmaf(k1312 * s3, s3, 0.25f * e * e);
+    const float yA = rcp(eps + bA), yB = rcp(eps + bB), yC = rcp(eps + bC), yD = rcp(eps + bD), yE = rcp(eps + bE);
+    up2(wz2(pk2(bA, bB), pk2(bC, bE), r2{yA, yB}, r2{yB, yD}, r2{yC, yE}, pk2(0.1f, 0.3f), sp2(0.6f), pk2(0.3f, 0.1f),
+            pk2(qA, qB), pk2(qB, qC), pk2(qC, qD)), L, R);
+}
+__device__ __forceinline__ void weno5_lr(float c0, float c1, float c2, float c3, float c4, float c5, float& L,
+                                         float& R) {
+    float bA, bB, bC, bD, bE;
+    weno5_lr(c0, c1, c2, c3, c4, c5, L, R, bA, bB, bC, bD, bE);
 }
 
 // f64::apply_floor with the FP64 pressure test skipped where an FP32
@@ -283,9 +291,130 @@ __device__ __forceinline__ void hllc_normal(float rL, float mnL, float mt1L, flo
     }
 }
 
-template <int D>
+// hllc_normal out of line, for the faces the packed form below leaves to it.
+__device__ __noinline__ inline void hllc_rare(float rL, float mnL, float mt1L, float mt2L, float EL, float rR, float mnR,
+                                              float mt1R, float mt2R, float ER, float g, float gm1, float gg, float* F) {
+    float Fr[5];
+    hllc_normal(rL, mnL, mt1L, mt2L, EL, rR, mnR, mt1R, mt2R, ER, g, gm1, gg, Fr);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) F[q] = Fr[q];
+}
+
+// P clamp, face energy (src/euler3d.jl:99-106) and HLLC (hllc_normal) of one
+// interface along axis D (a constant, or at run time) from its reconstructed
+// (rho, m, P) on both sides, with left and right as the two lanes of packed
+// instructions: each lane's operations are hllc_normal's, so are its bits.
+// Faces with a density at or below zero or a velocity above the cap take
+// hllc_normal itself.
+__device__ __forceinline__ void finish_face(const float (&c)[6][6], const float (&L)[5], const float (&R)[5], float g,
+                                            float gm1, float inv_gm1, float gg, int D, float F[5]) {
+    const float Pm = fmaxf(fmaxf(fmaxf(c[1][5], c[2][5]), c[3][5]), c[4][5]);   // values, so in any order
+    const float PL = fminf(fmaxf(L[4], 0.0f), fmaxf(c[0][5], Pm)), PR = fminf(fmaxf(R[4], 0.0f), fmaxf(Pm, c[5][5]));
+    const float rL = fmaxf(L[0], 1e-30f), rR = fmaxf(R[0], 1e-30f);
+    const f2 r = pk2(rL, rR), half = sp2(0.5f), i = pk2(rcp(rL), rcp(rR)), gm = sp2(gm1), gg2 = sp2(g);
+    const f2 mx = pk2(L[1], R[1]), my = pk2(L[2], R[2]), mz = pk2(L[3], R[3]);
+    const f2 cap = half * r * sp2(1e4f);
+    float x, y, capL, capR;
+    up2(cap, capL, capR);
+    // EL_from_P
+    up2(half * fma2(mz, mz, fma2(my, my, mx * mx)) * i, x, y);
+    f2 E = fma2(pk2(PL, PR), sp2(inv_gm1), pk2(fminf(x, capL), fminf(y, capR)));
+    // (normal, t1, t2) = (x, y, z), (y, x, z), (z, x, y)
+    const f2 mn = D == 0 ? mx : (D == 1 ? my : mz), mt1 = D == 0 ? my : mx, mt2 = D == 2 ? my : mz;
+    const f2 m2 = fma2(mt2, mt2, fma2(mt1, mt1, mn * mn));
+    float m2L, m2R, EL, ER, Fr[5];
+    up2(m2, m2L, m2R);
+    up2(E, EL, ER);
+    up2(r * r * sp2(1e4f), x, y);
+    if (L[0] <= 0.0f || R[0] <= 0.0f || m2L > x || m2R > y) {
+        float a1, a2, b1, b2, n1, n2;
+        up2(mn, n1, n2);
+        up2(mt1, a1, a2);
+        up2(mt2, b1, b2);
+        hllc_rare(L[0], n1, a1, b1, EL, R[0], n2, a2, b2, ER, g, gm1, gg, Fr);
+    } else {
+        up2(half * m2 * i, x, y);
+        const float KEL = fminf(x, capL), KER = fminf(y, capR);
+        const f2 KE = pk2(KEL, KER);
+        E = pk2(fmaxf(EL, KEL), fmaxf(ER, KER));
+        up2(E, EL, ER);
+        const f2 vn = mn * i, vt1 = mt1 * i, vt2 = mt2 * i;
+        const f2 p = gm * (E - KE);
+        float pL, pR, vnL, vnR;
+        up2(p, pL, pR);
+        up2(vn, vnL, vnR);
+        up2(gg2 * p * i, x, y);
+        const float csL = sqrtf(x), csR = sqrtf(y);
+        float SL, SR;
+        if (pL > 0.0f && pR > 0.0f) {
+            float r_avg = 0.5f * (rL + rR), cs_avg = 0.5f * (csL + csR);
+            float p_star = fmaxf(0.0f, fmaf(-0.5f * (vnR - vnL) * r_avg, cs_avg, 0.5f * (pL + pR)));
+            float qL = p_star > pL ? sqrtf(fmaf(gg, fdiv(p_star, pL) - 1.0f, 1.0f)) : 1.0f;
+            float qR = p_star > pR ? sqrtf(fmaf(gg, fdiv(p_star, pR) - 1.0f, 1.0f)) : 1.0f;
+            SL = fmaf(-csL, qL, vnL);
+            SR = fmaf(csR, qR, vnR);
+        } else {
+            SL = fminf(vnL - csL, vnR - csR);
+            SR = fmaxf(vnL + csL, vnR + csR);
+        }
+        const f2 S = pk2(SL, SR), Sv = S - vn, d = r * Sv;
+        float dL, dR, SvL, SvR, mnL, mnR;
+        up2(d, dL, dR);
+        up2(Sv, SvL, SvR);
+        up2(mn, mnL, mnR);
+        const float denom = dL - dR;
+        if (fabsf(denom) < 1e-36f) {
+            Fr[0] = Fr[1] = Fr[2] = Fr[3] = Fr[4] = 0.0f;
+        } else {
+            const float S_star = fdiv(fmaf(-mnR, SvR, fmaf(mnL, SvL, pR - pL)), denom);
+            const f2 Fmn = fma2(mn, vn, p), Ft1 = mt1 * vn, Ft2 = mt2 * vn, FE = (E + p) * vn;
+            float FmnL, FmnR, Ft1L, Ft1R, Ft2L, Ft2R, FEL, FER, t1L, t1R, t2L, t2R;
+            up2(Fmn, FmnL, FmnR);
+            up2(Ft1, Ft1L, Ft1R);
+            up2(Ft2, Ft2L, Ft2R);
+            up2(FE, FEL, FER);
+            up2(mt1, t1L, t1R);
+            up2(mt2, t2L, t2R);
+            if (SL >= 0.0f) {
+                Fr[0] = mnL; Fr[1] = FmnL; Fr[2] = Ft1L; Fr[3] = Ft2L; Fr[4] = FEL;
+            } else if (SR <= 0.0f) {
+                Fr[0] = mnR; Fr[1] = FmnR; Fr[2] = Ft1R; Fr[3] = Ft2R; Fr[4] = FER;
+            } else if (fmaxf(rL, rR) > 3.0f * fminf(rL, rR)) {
+                float inv = fdiv(1.0f, SR - SL), SLSR = SL * SR;
+                Fr[0] = fmaf(SLSR, rR - rL, fmaf(-SL, mnR, SR * mnL)) * inv;
+                Fr[1] = fmaf(SLSR, mnR - mnL, fmaf(-SL, FmnR, SR * FmnL)) * inv;
+                Fr[2] = fmaf(SLSR, t1R - t1L, fmaf(-SL, Ft1R, SR * Ft1L)) * inv;
+                Fr[3] = fmaf(SLSR, t2R - t2L, fmaf(-SL, Ft2R, SR * Ft2L)) * inv;
+                Fr[4] = fmaf(SLSR, ER - EL, fmaf(-SL, FER, SR * FEL)) * inv;
+            } else {
+                // the star flux of the upwind side, one instance for both
+                float v1L, v1R, v2L, v2R, iL, iR;
+                up2(vt1, v1L, v1R);
+                up2(vt2, v2L, v2R);
+                up2(i, iL, iR);
+                const bool left = S_star >= 0.0f;
+                const float Sk = left ? SL : SR, dk = left ? dL : dR, pk = left ? pL : pR, Ek = left ? EL : ER;
+                const float chi = fdiv(dk, Sk - S_star);
+                const float Es = fabsf(dk) > 1e-36f ? chi * fmaf(S_star - (left ? vnL : vnR), S_star + fdiv(pk, dk),
+                                                                 Ek * (left ? iL : iR)) : 0.0f;
+                Fr[0] = fmaf(Sk, chi - (left ? rL : rR), left ? mnL : mnR);
+                Fr[1] = fmaf(Sk, fmaf(chi, S_star, -(left ? mnL : mnR)), left ? FmnL : FmnR);
+                Fr[2] = fmaf(Sk, fmaf(chi, left ? v1L : v1R, -(left ? t1L : t1R)), left ? Ft1L : Ft1R);
+                Fr[3] = fmaf(Sk, fmaf(chi, left ? v2L : v2R, -(left ? t2L : t2R)), left ? Ft2L : Ft2R);
+                Fr[4] = fmaf(Sk, Es - Ek, left ? FEL : FER);
+            }
+        }
+    }
+    F[0] = Fr[0];
+    F[1] = D == 0 ? Fr[1] : Fr[2];
+    F[2] = D == 0 ? Fr[2] : (D == 1 ? Fr[1] : Fr[3]);
+    F[3] = D == 2 ? Fr[1] : Fr[3];
+    F[4] = Fr[4];
+}
+
+// One interface along axis D (a constant, or at run time).
 __device__ __forceinline__ void interface_flux(const float (&c)[6][6], float g, float gm1, float inv_gm1, float gg,
-                                               float F[5]) {
+                                               int D, float F[5]) {
     float L[5], R[5];
 #pragma unroll
     for (int q = 0; q < 4; q += 2) {
@@ -295,25 +424,8 @@ __device__ __forceinline__ void interface_flux(const float (&c)[6][6], float g, 
         up2(L2, L[q], L[q + 1]);
         up2(R2, R[q], R[q + 1]);
     }
-    float PL, PR;
-    weno5_lr(c[0][5], c[1][5], c[2][5], c[3][5], c[4][5], c[5][5], PL, PR);
-    float PmaxL = fmaxf(fmaxf(fmaxf(fmaxf(c[0][5], c[1][5]), c[2][5]), c[3][5]), c[4][5]);
-    float PmaxR = fmaxf(fmaxf(fmaxf(fmaxf(c[1][5], c[2][5]), c[3][5]), c[4][5]), c[5][5]);
-    PL = fminf(fmaxf(PL, 0.0f), PmaxL);
-    PR = fminf(fmaxf(PR, 0.0f), PmaxR);
-    float EL = EL_from_P(PL, L[0], L[1], L[2], L[3], inv_gm1);
-    float ER = EL_from_P(PR, R[0], R[1], R[2], R[3], inv_gm1);
-    float Fr[5];
-    if (D == 0) {
-        hllc_normal(L[0], L[1], L[2], L[3], EL, R[0], R[1], R[2], R[3], ER, g, gm1, gg, Fr);
-        F[0] = Fr[0]; F[1] = Fr[1]; F[2] = Fr[2]; F[3] = Fr[3]; F[4] = Fr[4];
-    } else if (D == 1) {
-        hllc_normal(L[0], L[2], L[1], L[3], EL, R[0], R[2], R[1], R[3], ER, g, gm1, gg, Fr);
-        F[0] = Fr[0]; F[1] = Fr[2]; F[2] = Fr[1]; F[3] = Fr[3]; F[4] = Fr[4];
-    } else {
-        hllc_normal(L[0], L[3], L[1], L[2], EL, R[0], R[3], R[1], R[2], ER, g, gm1, gg, Fr);
-        F[0] = Fr[0]; F[1] = Fr[2]; F[2] = Fr[3]; F[3] = Fr[1]; F[4] = Fr[4];
-    }
+    weno5_lr(c[0][5], c[1][5], c[2][5], c[3][5], c[4][5], c[5][5], L[4], R[4]);
+    finish_face(c, L, R, g, gm1, inv_gm1, gg, D, F);
 }
 
 }  // namespace f32

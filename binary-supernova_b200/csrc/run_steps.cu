@@ -61,6 +61,7 @@ struct State {
     int nx = 0, ny = 0, nz = 0, bc = 0, prec = 0, variant = -1;
     double dx = 0, dy = 0, dz = 0, gamma = 0, cfl = 0, rho_floor = 0, P_floor = 0, t_end = 0;
     double *A = nullptr, *B = nullptr;
+    const unsigned char* uni = nullptr;
     Dev* r = nullptr;
     cudaStream_t cap = nullptr;   // private stream used only to capture (the caller's may be the legacy stream)
     cudaEvent_t flag_ev[2] = {nullptr, nullptr};   // done-flag readbacks of the replay chunks
@@ -100,9 +101,15 @@ bsn_status rk3_prec(bsn_ctx* ctx, f64::StageArgs base, double* U, double dt, int
     double* B = (double*)slot(ctx, SLOT_B, bytes, &st); BSN_TRY(st);
     double* in[3] = {U, A, B};
     double* out[3] = {A, B, U};
+    base.Uin = U;
+    base.Un = U;
+    UniformTiles uni;
+    BSN_TRY(uniform_tiles_prepare(ctx, prec, base, uni));
+    BSN_TRY(uniform_tiles_find(ctx, prec, base, U, uni));
     for (int s = 0; s < 3; ++s) {
         f64::StageArgs a = base;
         a.Uin = in[s]; a.Un = U; a.Uout = out[s]; a.mode = 0;
+        uni.set(a, s);
         set_stage(a, s + 1, dt);
         BSN_TRY(stage_launch(ctx, prec, a));
     }
@@ -222,12 +229,10 @@ extern "C" bsn_status bsn_run_steps(bsn_ctx* ctx, double* U, int nx, int ny, int
     base.stiff_guard = ctx->stiff_guard;
     base.tune_class = TUNE_RUN;
     // autotune before any capture (it launches and times kernels)
-    auto tune = [&]() -> bsn_status {
-        bsn_status ts;
-        double* scratch = (double*)slot(ctx, SLOT_UN, bytes, &ts); BSN_TRY(ts);
-        return stage_autotune(ctx, precision, base, scratch);
-    };
+    UniformTiles uni;
+    auto tune = [&]() -> bsn_status { return uniform_tiles_prepare(ctx, precision, base, uni); };
     BSN_TRY(tune());
+    BSN_TRY(uniform_tiles_find(ctx, precision, base, U, uni));
     int variant = tile_code(ctx, precision, base);
 
     init_kernel<<<1, 1, 0, ctx->stream>>>(r, *t_inout);
@@ -237,7 +242,26 @@ extern "C" bsn_status bsn_run_steps(bsn_ctx* ctx, double* U, int nx, int ny, int
     bool same = S->exec && S->U == U && S->nx == nx && S->ny == ny && S->nz == nz && S->dx == dx && S->dy == dy &&
                 S->dz == dz && S->gamma == gamma && S->cfl == cfl && S->bc == bc && S->rho_floor == rho_floor &&
                 S->P_floor == P_floor && S->prec == precision && S->t_end == t_end && S->variant == variant &&
-                S->A == A && S->B == B && S->r == r;
+                S->A == A && S->B == B && S->r == r && S->uni == (uni.on ? uni.f[0] : nullptr);
+    auto body = [&]() -> bsn_status {   // one step
+        dt_kernel<<<1, 1, 0, ctx->stream>>>(r, cfl, t_end);
+        BSN_TRY(launch_check(ctx, "run_dt_kernel"));
+        double* in[3] = {U, A, B};
+        double* out[3] = {A, B, U};
+        for (int s = 0; s < 3; ++s) {
+            f64::StageArgs a = base;
+            a.Uin = in[s]; a.Un = U; a.Uout = out[s]; a.mode = 0;
+            uni.set(a, s);
+            set_stage(a, s + 1, 0.0);
+            a.dt_dev = &r->dt;
+            a.done_dev = &r->done;
+            if (s == 2) { a.cfl_max = &r->smax; a.cfl_nan = &r->nanflag; }
+            BSN_TRY(stage_launch(ctx, precision, a));
+        }
+        BSN_TRY(f64_ghost_combine(ctx, U, B, nullptr, nx, ny, nz, bc, 0.0, &r->dt, &r->done));
+        advance_kernel<<<1, 1, 0, ctx->stream>>>(r);
+        return launch_check(ctx, "run_advance_kernel");
+    };
     auto capture = [&]() -> bsn_status {
         release(S);
         if (!S->cap) BSN_CUDA(ctx, cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking));
@@ -251,25 +275,7 @@ extern "C" bsn_status bsn_run_steps(bsn_ctx* ctx, double* U, int nx, int ny, int
             cudaError_t be = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
             if (be != cudaSuccess) { ctx->stream = user; ctx->profiling = prof; return cuda_check(ctx, be, "cudaStreamBeginCapture"); }
         }
-        bsn_status cst = BSN_OK;
-        dt_kernel<<<1, 1, 0, ctx->stream>>>(r, cfl, t_end);
-        cst = launch_check(ctx, "run_dt_kernel");
-        double* in[3] = {U, A, B};
-        double* out[3] = {A, B, U};
-        for (int s = 0; s < 3 && cst == BSN_OK; ++s) {
-            f64::StageArgs a = base;
-            a.Uin = in[s]; a.Un = U; a.Uout = out[s]; a.mode = 0;
-            set_stage(a, s + 1, 0.0);
-            a.dt_dev = &r->dt;
-            a.done_dev = &r->done;
-            if (s == 2) { a.cfl_max = &r->smax; a.cfl_nan = &r->nanflag; }
-            cst = stage_launch(ctx, precision, a);
-        }
-        if (cst == BSN_OK) cst = f64_ghost_combine(ctx, U, B, nullptr, nx, ny, nz, bc, 0.0, &r->dt, &r->done);
-        if (cst == BSN_OK) {
-            advance_kernel<<<1, 1, 0, ctx->stream>>>(r);
-            cst = launch_check(ctx, "run_advance_kernel");
-        }
+        bsn_status cst = body();
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
         ctx->stream = user;
@@ -283,23 +289,29 @@ extern "C" bsn_status bsn_run_steps(bsn_ctx* ctx, double* U, int nx, int ny, int
         S->U = U; S->nx = nx; S->ny = ny; S->nz = nz; S->dx = dx; S->dy = dy; S->dz = dz; S->gamma = gamma;
         S->cfl = cfl; S->bc = bc; S->rho_floor = rho_floor; S->P_floor = P_floor; S->prec = precision;
         S->t_end = t_end; S->variant = variant; S->A = A; S->B = B; S->r = r;
+        S->uni = uni.on ? uni.f[0] : nullptr;
         return BSN_OK;
     };
-    if (!same) BSN_TRY(capture());
+    const bool direct = !same && n_steps <= kDirectSteps;
+    if (!same && !direct) BSN_TRY(capture());
     double* h = (double*)pinned(ctx, 128, &st); BSN_TRY(st);
     // replays after t_end are no-ops: with t_end, stop once the device says done
     const bool settle = n_steps >= 2 && !tile_settled(ctx, TUNE_RUN, precision);
-    BSN_TRY(graph_replay(ctx, S->exec, S->kernels, settle ? 1 : n_steps, t_end > 0.0, &r->done, S->flag_ev,
-                         (volatile int*)(h + 8)));
+    auto advance = [&](int n) -> bsn_status {
+        if (direct) return launch_steps(ctx, body, n);
+        return graph_replay(ctx, S->exec, S->kernels, n, t_end > 0.0, &r->done, S->flag_ev,
+                         (volatile int*)(h + 8));
+    };
+    BSN_TRY(advance(settle ? 1 : n_steps));
     if (settle) {   // the tile re-timed on the state after the first step
         BSN_TRY(tile_retime(ctx, TUNE_RUN, precision, tune));
         if (tile_code(ctx, precision, base) != variant) {
             variant = tile_code(ctx, precision, base);
             BSN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            BSN_TRY(capture());
+            if (!direct) BSN_TRY(capture());
         }
-        BSN_TRY(graph_replay(ctx, S->exec, S->kernels, n_steps - 1, t_end > 0.0, &r->done, S->flag_ev,
-                             (volatile int*)(h + 8)));
+        BSN_TRY(uniform_tiles_find(ctx, precision, base, U, uni));   // of the new tile, or over the re-timing's use
+        BSN_TRY(advance(n_steps - 1));
     }
     BSN_CUDA(ctx, cudaMemcpyAsync(h, r, sizeof(Dev), cudaMemcpyDeviceToHost, ctx->stream));
     BSN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

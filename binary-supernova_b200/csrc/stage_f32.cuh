@@ -13,7 +13,7 @@ namespace tile {
 
 struct F32Physics {
     using real = float;
-    static constexpr bool kStiffFallback = false;
+    static constexpr bool kDeferred = false;
     static constexpr int kCols = 5;                  // rho, m, P: the epilogue reloads the FP64 state
     static constexpr bool kCenterFromSmem = false;  // smem holds FP32 copies: reload FP64 state
     static constexpr bool kWarpFaces = false;
@@ -40,9 +40,9 @@ struct F32Physics {
         P = pressure(w, k);
         return true;
     }
-    template <int D>
-    __device__ static void flux(const float (&c)[6][6], const Consts& k, float F[5]) {
-        f32::interface_flux<D>(c, k.g, k.gm1, k.inv_gm1, k.gg, F);
+    __device__ __forceinline__ static bool flux(const float (&c)[6][6], const Consts& k, int D, float F[5]) {
+        f32::interface_flux(c, k.g, k.gm1, k.inv_gm1, k.gg, D, F);
+        return false;
     }
 };
 
@@ -52,7 +52,11 @@ struct F32Physics {
 // A.stiff_guard is set: the coupled driver loops with sinks (near-vacuum
 // cells beside dense gas), or any loop on request.
 struct F32Guarded : F32Physics {
-    static constexpr bool kStiffFallback = true;
+    static constexpr bool kDeferred = true;
+    __device__ __forceinline__ static bool flux(const float (&c)[6][6], const Consts& k, int D, float F[5]) {
+        if (stiff_stencil(c)) return true;
+        return F32Physics::flux(c, k, D, F);
+    }
 };
 
 }  // namespace tile

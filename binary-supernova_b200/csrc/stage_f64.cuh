@@ -68,7 +68,7 @@ struct StageArgs {
     // others here; the learned launch then does the listed blocks
     int learned_split;            // learned stages split (uniform-grid entry points; off elsewhere)
     int* split_list;              // block index bx + gx (by + gy bz)
-    unsigned int* split_count;
+    unsigned int* split_count;    // entries, and the queue counter of the launch that walks them
     const BHSrc* bh_dev;     // non-null: gravity sources read on the device (device-resident driver loop)
     const SinkSrc* sk_dev;   // non-null: sink sources read on the device
     // relaxation sources (src/relax_ic.jl): rotating frame at rot_omega,
@@ -96,6 +96,17 @@ struct StageArgs {
     int k0;
     const double* phi_lo;
     const double* phi_hi;
+    // uniform tiles: one byte per tile of the launch's tile shape, 1 where every
+    // active cell of the tile holds the same five words, of the stage's input
+    // and base state (read) and of its result (written); null: not kept.  With
+    // them a stage is two launches: uniform_stage_kernel does the tiles whose
+    // result is one cell and lists the others, which the stage kernel walks.
+    const unsigned char* uni_in;
+    const unsigned char* uni_un;
+    unsigned char* uni_out;
+    int* list;                    // block index bx + gx (by + gy bz)
+    unsigned int* list_count;     // entries, and the queue counter of the launch that walks them
+    unsigned int* list_zero;      // the next stage's list_count, cleared by this one
     // the driver loop this stage belongs to (TUNE_* in stage_launch.cuh): the
     // autotuner keeps one tile choice per driver and grid, so a driver's
     // choice is timed on its own stage arguments and grid contents

@@ -22,6 +22,8 @@ size_t learned_split_bytes(int nx, int ny, int nz);
 int f64_variant_count();
 TileVariant f64_variant(int idx);
 bsn_status f64_launch_variant(bsn_ctx* ctx, int idx, const f64::StageArgs& A);
+bsn_status f64_launch_variant_lo(bsn_ctx* ctx, int idx, const f64::StageArgs& A);
+bsn_status f64_launch_variant_hi(bsn_ctx* ctx, int idx, const f64::StageArgs& A);
 int f32_variant_count();
 TileVariant f32_variant(int idx);
 bsn_status f32_launch_variant(bsn_ctx* ctx, int idx, const f64::StageArgs& A);
@@ -30,6 +32,8 @@ TileVariant learned_variant(int idx);
 bsn_status learned_launch_variant(bsn_ctx* ctx, int idx, const f64::StageArgs& A);
 // batched (several grids in one persistent launch) counterparts
 bsn_status f64_launch_batch_variant(bsn_ctx* ctx, int idx, const f64::StageBatch& B);
+bsn_status f64_launch_batch_variant_lo(bsn_ctx* ctx, int idx, const f64::StageBatch& B);
+bsn_status f64_launch_batch_variant_hi(bsn_ctx* ctx, int idx, const f64::StageBatch& B);
 bsn_status f32_launch_batch_variant(bsn_ctx* ctx, int idx, const f64::StageBatch& B);
 bsn_status learned_launch_batch_variant(bsn_ctx* ctx, int idx, const f64::StageBatch& B);
 
@@ -55,6 +59,33 @@ bsn_status stage_launch_batch(bsn_ctx* ctx, int precision, const f64::StageBatch
 // Autotune explicitly (must not run during stream capture): times every
 // variant on stage-1 work writing to `scratch` and records the fastest.
 bsn_status stage_autotune(bsn_ctx* ctx, int precision, const f64::StageArgs& probe, double* scratch);
+// The same for drivers whose stages run over several grids in one launch: one
+// choice for the n grids, timed in one launch over all of them.
+bsn_status stage_autotune_batch(bsn_ctx* ctx, int precision, const f64::StageArgs* probes, double* const* scratch,
+                                int n);
+
+// Uniform tiles of a step's three arrays (StageArgs::uni_*; stage_tile.cuh):
+// U, and the results of stages 1 and 2.  on = false where they are not kept.
+struct UniformTiles {
+    unsigned char* f[3] = {nullptr, nullptr, nullptr};
+    int* list = nullptr;              // the tiles a stage leaves to the stage kernel
+    unsigned int* count = nullptr;    // list count and queue counter of each stage
+    bool on = false;
+    void set(f64::StageArgs& a, int s) const {   // stage s = 0, 1, 2
+        if (!on) return;
+        a.uni_in = f[s];
+        a.uni_un = f[0];
+        a.uni_out = f[(s + 1) % 3];
+        a.list = list;
+        a.list_count = count + 2 * s;
+        a.list_zero = count + 2 * ((s + 1) % 3);
+    }
+};
+// Room for them, and the tile choice of base's grid (autotuned where it may).
+bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int precision, const f64::StageArgs& base, UniformTiles& t);
+// Those of U, for the tile choice of base's grid, and cleared counts.
+bsn_status uniform_tiles_find(bsn_ctx* ctx, int precision, const f64::StageArgs& base, const double* U,
+                              const UniformTiles& t);
 
 // Device loops tune on the state they are first called with.  From an
 // initial condition (gas at rest) every tile variant can time within a
