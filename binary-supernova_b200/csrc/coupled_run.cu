@@ -376,6 +376,57 @@ extern "C" bsn_status bsn_coupled_run_steps(bsn_ctx* ctx, double* U, bsn_bh* bhs
                 S->f_sink == f_sink && S->rho_floor == rho_floor && S->P_floor == P_floor &&
                 S->t_on == t_bh2_sink_on && S->rho_min == rho_sink_min && S->t_end == t_end &&
                 S->diag_cap == diag_cap && memcmp(S->ptrs, ptrs, sizeof(ptrs)) == 0;
+    auto body = [&]() -> bsn_status {
+        dt_kernel<<<1, 1, 0, ctx->stream>>>(r, cfl, t_end, dt_max);
+        BSN_TRY(launch_check(ctx, "coupled_dt_kernel"));
+        // gas force on every BH from the start-of-step state, then the orbit
+        for (int i = 0; i < nbh; ++i) {
+            gas_force_kernel<<<blocks, 256, 0, ctx->stream>>>(U, nx, ny, nz, dx, dx, dx, x0, y0, z0, r, i, part,
+                                                              Box{{1, 1, 1}, {0, 0, 0}});
+            BSN_TRY(launch_check(ctx, "coupled_gas_force_kernel"));
+            gas_force_finish<<<1, 256, 0, ctx->stream>>>(part, blocks, r, i);
+            BSN_TRY(launch_check(ctx, "coupled_gas_force_finish"));
+        }
+        if (evolve_orbit && nbh > 0) {
+            nbody_kernel<<<1, 32, 0, ctx->stream>>>(r);
+            BSN_TRY(launch_check(ctx, "coupled_nbody_kernel"));
+        }
+        fill_kernel<<<1, 32, 0, ctx->stream>>>(r, f_sink, torque_free, rho_sink_min, t_bh2_sink_on);
+        BSN_TRY(launch_check(ctx, "coupled_fill_kernel"));
+        // SSP-RK3 with the sources in the driver's order (stage epilogue)
+        double* in[3] = {U, A, B};
+        double* out[3] = {A, B, U};
+        for (int s = 0; s < 3; ++s) {
+            f64::StageArgs a = base;
+            a.Uin = in[s]; a.Un = U; a.Uout = out[s]; a.mode = 0;
+            set_stage(a, s + 1, 0.0);
+            a.dt_dev = &r->dt;
+            a.done_dev = &r->done;
+            if (nbh > 0) { a.use_bh = 1; a.bh_dev = &r->bsrc; a.use_sink = 1; a.sk_dev = &r->ssrc; }
+            if (self_gravity) {
+                if (precision == PREC_F64) BSN_TRY(poisson_from_state(ctx, in[s], nx, ny, nz, dx, dx, dx, rho_floor, phi));
+                else BSN_TRY(poisson_from_state_f32(ctx, in[s], nx, ny, nz, dx, dx, dx, rho_floor, phi));
+                a.phi = phi; a.use_sg = 1;
+            }
+            if (s == 2) { a.cfl_max = &r->smax; a.cfl_nan = &r->nanflag; }
+            a.ledger = &r->led[0][s][0];
+            a.led_bnd = 1;
+            BSN_TRY(stage_launch(ctx, precision, a));
+        }
+        BSN_TRY(f64_ledger_fold(ctx, &r->led[0][0][0], r->led_tot, &r->dt, &r->done));
+        BSN_TRY(f64_ghost_combine(ctx, U, B, nullptr, nx, ny, nz, BSN_BC_OUTFLOW, 0.0, &r->dt, &r->done));
+        for (int i = 0; i < nbh; ++i) {
+            accrete_kernel<<<1, 256, 0, ctx->stream>>>(U, nx, ny, nz, dx, dx, dx, x0, y0, z0, r, i, f_sink,
+                                                      rho_sink_min);
+            BSN_TRY(launch_check(ctx, "coupled_accrete_kernel"));
+        }
+        advance_kernel<<<1, 1, 0, ctx->stream>>>(r);
+        BSN_TRY(launch_check(ctx, "coupled_advance_kernel"));
+        if (diag_out)   // the driver's diagnostics of the end-of-step state (BHs after accretion)
+            BSN_TRY(diag::launch(ctx, U, nx, ny, nz, dx, dx, dx, x0, y0, z0, r->bh, &r->nbh, nbh, gamma, dpart,
+                                 diag_out, &r->t, &r->dt, &r->steps, &r->done, diag_cap, r->led_tot));
+        return BSN_OK;
+    };
     auto capture = [&]() -> bsn_status {
         S->release();
         if (!S->cap) BSN_CUDA(ctx, cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking));
@@ -386,57 +437,6 @@ extern "C" bsn_status bsn_coupled_run_steps(bsn_ctx* ctx, double* U, bsn_bh* bhs
         ctx->stream = S->cap;
         cudaError_t be = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
         if (be != cudaSuccess) { ctx->stream = user; ctx->profiling = prof; return cuda_check(ctx, be, "cudaStreamBeginCapture"); }
-        auto body = [&]() -> bsn_status {
-            dt_kernel<<<1, 1, 0, ctx->stream>>>(r, cfl, t_end, dt_max);
-            BSN_TRY(launch_check(ctx, "coupled_dt_kernel"));
-            // gas force on every BH from the start-of-step state, then the orbit
-            for (int i = 0; i < nbh; ++i) {
-                gas_force_kernel<<<blocks, 256, 0, ctx->stream>>>(U, nx, ny, nz, dx, dx, dx, x0, y0, z0, r, i, part,
-                                                                  Box{{1, 1, 1}, {0, 0, 0}});
-                BSN_TRY(launch_check(ctx, "coupled_gas_force_kernel"));
-                gas_force_finish<<<1, 256, 0, ctx->stream>>>(part, blocks, r, i);
-                BSN_TRY(launch_check(ctx, "coupled_gas_force_finish"));
-            }
-            if (evolve_orbit && nbh > 0) {
-                nbody_kernel<<<1, 32, 0, ctx->stream>>>(r);
-                BSN_TRY(launch_check(ctx, "coupled_nbody_kernel"));
-            }
-            fill_kernel<<<1, 32, 0, ctx->stream>>>(r, f_sink, torque_free, rho_sink_min, t_bh2_sink_on);
-            BSN_TRY(launch_check(ctx, "coupled_fill_kernel"));
-            // SSP-RK3 with the sources in the driver's order (stage epilogue)
-            double* in[3] = {U, A, B};
-            double* out[3] = {A, B, U};
-            for (int s = 0; s < 3; ++s) {
-                f64::StageArgs a = base;
-                a.Uin = in[s]; a.Un = U; a.Uout = out[s]; a.mode = 0;
-                set_stage(a, s + 1, 0.0);
-                a.dt_dev = &r->dt;
-                a.done_dev = &r->done;
-                if (nbh > 0) { a.use_bh = 1; a.bh_dev = &r->bsrc; a.use_sink = 1; a.sk_dev = &r->ssrc; }
-                if (self_gravity) {
-                    if (precision == PREC_F64) BSN_TRY(poisson_from_state(ctx, in[s], nx, ny, nz, dx, dx, dx, rho_floor, phi));
-                    else BSN_TRY(poisson_from_state_f32(ctx, in[s], nx, ny, nz, dx, dx, dx, rho_floor, phi));
-                    a.phi = phi; a.use_sg = 1;
-                }
-                if (s == 2) { a.cfl_max = &r->smax; a.cfl_nan = &r->nanflag; }
-                a.ledger = &r->led[0][s][0];
-                a.led_bnd = 1;
-                BSN_TRY(stage_launch(ctx, precision, a));
-            }
-            BSN_TRY(f64_ledger_fold(ctx, &r->led[0][0][0], r->led_tot, &r->dt, &r->done));
-            BSN_TRY(f64_ghost_combine(ctx, U, B, nullptr, nx, ny, nz, BSN_BC_OUTFLOW, 0.0, &r->dt, &r->done));
-            for (int i = 0; i < nbh; ++i) {
-                accrete_kernel<<<1, 256, 0, ctx->stream>>>(U, nx, ny, nz, dx, dx, dx, x0, y0, z0, r, i, f_sink,
-                                                          rho_sink_min);
-                BSN_TRY(launch_check(ctx, "coupled_accrete_kernel"));
-            }
-            advance_kernel<<<1, 1, 0, ctx->stream>>>(r);
-            BSN_TRY(launch_check(ctx, "coupled_advance_kernel"));
-            if (diag_out)   // the driver's diagnostics of the end-of-step state (BHs after accretion)
-                BSN_TRY(diag::launch(ctx, U, nx, ny, nz, dx, dx, dx, x0, y0, z0, r->bh, &r->nbh, nbh, gamma, dpart,
-                                     diag_out, &r->t, &r->dt, &r->steps, &r->done, diag_cap, r->led_tot));
-            return BSN_OK;
-        };
         bsn_status cst = body();
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
@@ -457,19 +457,23 @@ extern "C" bsn_status bsn_coupled_run_steps(bsn_ctx* ctx, double* U, bsn_bh* bhs
         memcpy(S->ptrs, ptrs, sizeof(ptrs));
         return BSN_OK;
     };
-    if (!same) BSN_TRY(capture());
+    const bool direct = !same && n_steps <= kDirectSteps;
+    if (!same && !direct) BSN_TRY(capture());
     const bool settle = n_steps >= 2 && !tile_settled(ctx, TUNE_COUPLED, precision);
-    BSN_TRY(graph_replay(ctx, S->exec, S->kernels, settle ? 1 : n_steps, t_end > 0.0, &r->done, S->ev,
-                         (volatile int*)((char*)h + sizeof(Dev))));
+    auto advance = [&](int n) -> bsn_status {
+        if (direct) return launch_steps(ctx, body, n);
+        return graph_replay(ctx, S->exec, S->kernels, n, t_end > 0.0, &r->done, S->ev,
+                         (volatile int*)((char*)h + sizeof(Dev)));
+    };
+    BSN_TRY(advance(settle ? 1 : n_steps));
     if (settle) {   // the tile re-timed on the state after the first step
         BSN_TRY(tile_retime(ctx, TUNE_COUPLED, precision, tune));
         if (tile_code(ctx, precision, base) != variant) {
             variant = tile_code(ctx, precision, base);
             BSN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            BSN_TRY(capture());
+            if (!direct) BSN_TRY(capture());
         }
-        BSN_TRY(graph_replay(ctx, S->exec, S->kernels, n_steps - 1, t_end > 0.0, &r->done, S->ev,
-                             (volatile int*)((char*)h + sizeof(Dev))));
+        BSN_TRY(advance(n_steps - 1));
     }
     BSN_CUDA(ctx, cudaMemcpyAsync(h, r, sizeof(Dev), cudaMemcpyDeviceToHost, ctx->stream));
     BSN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -585,11 +589,14 @@ extern "C" bsn_status bsn_coupled_nested_run_steps(bsn_ctx* ctx, const bsn_fmr2*
             fill_kernel<<<1, 32, 0, ctx->stream>>>(r, f_sink, torque_free, rho_sink_min, t_bh2_sink_on);
             BSN_TRY(launch_check(ctx, "coupled_fill_kernel"));
         }
+        f64::StageArgs p[NMAXL];
+        double* out[NMAXL];
         for (int l = 0; l < nl; ++l) {
-            f64::StageArgs p = plan.base[l];
-            p.Uin = plan.L[l].U; p.dt_dev = nullptr; p.done_dev = nullptr; p.use_reg = 0; p.use_bnd = 0; p.Gh = nullptr;
-            BSN_TRY(stage_autotune(ctx, precision, p, plan.L[l].A));
+            p[l] = plan.base[l];
+            p[l].Uin = plan.L[l].U; p[l].Gh = nullptr;
+            out[l] = plan.L[l].A;
         }
+        BSN_TRY(stage_autotune_batch(ctx, precision, p, out, nl));
         for (int l = 0; l < nl; ++l) tiles[l] = tile_code(ctx, precision, plan.base[l]);
         return BSN_OK;
     };
@@ -604,6 +611,58 @@ extern "C" bsn_status bsn_coupled_nested_run_steps(bsn_ctx* ctx, const bsn_fmr2*
                 memcmp(S->key_pairs.data(), pairs, sizeof(bsn_fmr2) * npairs) == 0 && S->prec == precision &&
                 S->sg == self_gravity && S->cfl == cfl && S->t_end == t_end &&
                 memcmp(S->tiles, tiles, sizeof(tiles)) == 0 && S->key_base == S->arena.base && S->key_extra == extra;
+    auto body = [&]() -> bsn_status {
+        for (int l = 0; l < nl; ++l) {
+            const NLevel& v = plan.L[l];
+            BSN_TRY(f64_cfl_fold(ctx, v.U, v.nx, v.ny, v.nz, v.dx, v.dy, v.dz, plan.gamma, &plan.d->sm[l],
+                                 &plan.d->nan[l]));
+        }
+        n_dt_kernel<<<1, 1, 0, ctx->stream>>>(plan.d, cfl, plan.R, t_end, dt_max);
+        BSN_TRY(launch_check(ctx, "fmrN_dt_kernel"));
+        nested_sync_kernel<<<1, 1, 0, ctx->stream>>>(r, plan.d);
+        BSN_TRY(launch_check(ctx, "coupled_nested_sync_kernel"));
+        // gas force on every BH from the composite of the levels
+        for (int i = 0; i < nbh; ++i) {
+            for (int l = 0; l < nl; ++l) {
+                const NLevel& v = plan.L[l];
+                Box skip{{1, 1, 1}, {0, 0, 0}};
+                if (l < nl - 1)
+                    for (int d = 0; d < 3; ++d) {
+                        skip.lo[d] = plan.P[l].G.lo[d] - 1;
+                        skip.hi[d] = plan.P[l].G.hi[d] - 1;
+                    }
+                gas_force_kernel<<<blocks, 256, 0, ctx->stream>>>(v.U, v.nx, v.ny, v.nz, v.dx, v.dy, v.dz, ox[l],
+                                                                  oy[l], oz[l], r, i, part + 6 * blocks * l, skip);
+                BSN_TRY(launch_check(ctx, "coupled_gas_force_kernel"));
+            }
+            gas_force_finish<<<1, 256, 0, ctx->stream>>>(part, blocks * nl, r, i);
+            BSN_TRY(launch_check(ctx, "coupled_gas_force_finish"));
+        }
+        if (evolve_orbit && nbh > 0) {
+            nbody_kernel<<<1, 32, 0, ctx->stream>>>(r);
+            BSN_TRY(launch_check(ctx, "coupled_nbody_kernel"));
+        }
+        fill_kernel<<<1, 32, 0, ctx->stream>>>(r, f_sink, torque_free, rho_sink_min, t_bh2_sink_on);
+        BSN_TRY(launch_check(ctx, "coupled_fill_kernel"));
+        BSN_TRY(plan.step());
+        for (int i = 0; i < nbh; ++i) {
+            accrete_kernel<<<1, 256, 0, ctx->stream>>>(fin.U, fin.nx, fin.ny, fin.nz, fin.dx, fin.dy, fin.dz,
+                                                      ox[nl - 1], oy[nl - 1], oz[nl - 1], r, i, f_sink,
+                                                      rho_sink_min);
+            BSN_TRY(launch_check(ctx, "coupled_accrete_kernel"));
+        }
+        n_advance_kernel<<<1, 1, 0, ctx->stream>>>(plan.d);
+        BSN_TRY(launch_check(ctx, "fmrN_advance_kernel"));
+        nested_sync_kernel<<<1, 1, 0, ctx->stream>>>(r, plan.d);
+        BSN_TRY(launch_check(ctx, "coupled_nested_sync_kernel"));
+        if (diag_out) {
+            const NLevel& v = plan.L[0];
+            BSN_TRY(diag::launch(ctx, v.U, v.nx, v.ny, v.nz, v.dx, v.dy, v.dz, x0, y0, z0, r->bh, &r->nbh, nbh,
+                                 plan.gamma, dpart, diag_out, &r->t, &r->dt, &r->steps, &r->done, diag_cap,
+                                 r->led_tot));
+        }
+        return BSN_OK;
+    };
     auto capture = [&]() -> bsn_status {
         S->release();
         if (!S->cap) BSN_CUDA(ctx, cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking));
@@ -614,58 +673,6 @@ extern "C" bsn_status bsn_coupled_nested_run_steps(bsn_ctx* ctx, const bsn_fmr2*
         ctx->stream = S->cap;
         cudaError_t be = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
         if (be != cudaSuccess) { ctx->stream = user; ctx->profiling = prof; return cuda_check(ctx, be, "cudaStreamBeginCapture"); }
-        auto body = [&]() -> bsn_status {
-            for (int l = 0; l < nl; ++l) {
-                const NLevel& v = plan.L[l];
-                BSN_TRY(f64_cfl_fold(ctx, v.U, v.nx, v.ny, v.nz, v.dx, v.dy, v.dz, plan.gamma, &plan.d->sm[l],
-                                     &plan.d->nan[l]));
-            }
-            n_dt_kernel<<<1, 1, 0, ctx->stream>>>(plan.d, cfl, plan.R, t_end, dt_max);
-            BSN_TRY(launch_check(ctx, "fmrN_dt_kernel"));
-            nested_sync_kernel<<<1, 1, 0, ctx->stream>>>(r, plan.d);
-            BSN_TRY(launch_check(ctx, "coupled_nested_sync_kernel"));
-            // gas force on every BH from the composite of the levels
-            for (int i = 0; i < nbh; ++i) {
-                for (int l = 0; l < nl; ++l) {
-                    const NLevel& v = plan.L[l];
-                    Box skip{{1, 1, 1}, {0, 0, 0}};
-                    if (l < nl - 1)
-                        for (int d = 0; d < 3; ++d) {
-                            skip.lo[d] = plan.P[l].G.lo[d] - 1;
-                            skip.hi[d] = plan.P[l].G.hi[d] - 1;
-                        }
-                    gas_force_kernel<<<blocks, 256, 0, ctx->stream>>>(v.U, v.nx, v.ny, v.nz, v.dx, v.dy, v.dz, ox[l],
-                                                                      oy[l], oz[l], r, i, part + 6 * blocks * l, skip);
-                    BSN_TRY(launch_check(ctx, "coupled_gas_force_kernel"));
-                }
-                gas_force_finish<<<1, 256, 0, ctx->stream>>>(part, blocks * nl, r, i);
-                BSN_TRY(launch_check(ctx, "coupled_gas_force_finish"));
-            }
-            if (evolve_orbit && nbh > 0) {
-                nbody_kernel<<<1, 32, 0, ctx->stream>>>(r);
-                BSN_TRY(launch_check(ctx, "coupled_nbody_kernel"));
-            }
-            fill_kernel<<<1, 32, 0, ctx->stream>>>(r, f_sink, torque_free, rho_sink_min, t_bh2_sink_on);
-            BSN_TRY(launch_check(ctx, "coupled_fill_kernel"));
-            BSN_TRY(plan.step());
-            for (int i = 0; i < nbh; ++i) {
-                accrete_kernel<<<1, 256, 0, ctx->stream>>>(fin.U, fin.nx, fin.ny, fin.nz, fin.dx, fin.dy, fin.dz,
-                                                          ox[nl - 1], oy[nl - 1], oz[nl - 1], r, i, f_sink,
-                                                          rho_sink_min);
-                BSN_TRY(launch_check(ctx, "coupled_accrete_kernel"));
-            }
-            n_advance_kernel<<<1, 1, 0, ctx->stream>>>(plan.d);
-            BSN_TRY(launch_check(ctx, "fmrN_advance_kernel"));
-            nested_sync_kernel<<<1, 1, 0, ctx->stream>>>(r, plan.d);
-            BSN_TRY(launch_check(ctx, "coupled_nested_sync_kernel"));
-            if (diag_out) {
-                const NLevel& v = plan.L[0];
-                BSN_TRY(diag::launch(ctx, v.U, v.nx, v.ny, v.nz, v.dx, v.dy, v.dz, x0, y0, z0, r->bh, &r->nbh, nbh,
-                                     plan.gamma, dpart, diag_out, &r->t, &r->dt, &r->steps, &r->done, diag_cap,
-                                     r->led_tot));
-            }
-            return BSN_OK;
-        };
         bsn_status cst = body();
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
@@ -684,18 +691,22 @@ extern "C" bsn_status bsn_coupled_nested_run_steps(bsn_ctx* ctx, const bsn_fmr2*
         S->key_extra = extra;
         return BSN_OK;
     };
-    if (!same) BSN_TRY(capture());
+    const bool direct = !same && n_steps <= kDirectSteps;
+    if (!same && !direct) BSN_TRY(capture());
     const bool settle = n_steps >= 2 && !tile_settled(ctx, TUNE_NESTED, precision);
-    BSN_TRY(graph_replay(ctx, S->exec, S->kernels, settle ? 1 : n_steps, t_end > 0.0, plan.done, S->ev,
-                         (volatile int*)((char*)h + sizeof(Dev) + sizeof(NDev))));
+    auto advance = [&](int n) -> bsn_status {
+        if (direct) return launch_steps(ctx, body, n);
+        return graph_replay(ctx, S->exec, S->kernels, n, t_end > 0.0, plan.done, S->ev,
+                         (volatile int*)((char*)h + sizeof(Dev) + sizeof(NDev)));
+    };
+    BSN_TRY(advance(settle ? 1 : n_steps));
     if (settle) {   // the tiles re-timed on the state after the first step
         BSN_TRY(tile_retime(ctx, TUNE_NESTED, precision, tune));
-        if (memcmp(S->tiles, tiles, sizeof(tiles)) != 0) {
+        if (!direct && memcmp(S->tiles, tiles, sizeof(tiles)) != 0) {
             BSN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             BSN_TRY(capture());
         }
-        BSN_TRY(graph_replay(ctx, S->exec, S->kernels, n_steps - 1, t_end > 0.0, plan.done, S->ev,
-                             (volatile int*)((char*)h + sizeof(Dev) + sizeof(NDev))));
+        BSN_TRY(advance(n_steps - 1));
     }
     NDev* hn = (NDev*)((char*)h + sizeof(Dev));
     BSN_CUDA(ctx, cudaMemcpyAsync(h, r, sizeof(Dev), cudaMemcpyDeviceToHost, ctx->stream));

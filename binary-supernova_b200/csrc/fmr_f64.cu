@@ -551,13 +551,13 @@ bsn_status fmr3d_run(bsn_ctx* ctx, const bsn_fmr2* g, double cfl, int prec, int 
     // tile choices before any capture (the autotuner launches and times)
     auto tune = [&]() -> bsn_status {
         bsn_status ts;
-        double* scratch = (double*)slot(ctx, SLOT_UN, sizeof(double) * std::max(C.nelem(), F.nelem()), &ts);
+        double* scratch = (double*)slot(ctx, SLOT_UN, sizeof(double) * (C.nelem() + F.nelem()), &ts);
         BSN_TRY(ts);
-        f64::StageArgs pc = cb, pf = fb;
-        pc.Uin = g->Uc; pc.dt_dev = nullptr; pc.done_dev = nullptr; pc.use_reg = 0;
-        pf.Uin = g->Uf; pf.dt_dev = nullptr; pf.done_dev = nullptr; pf.use_bnd = 0; pf.Gh = nullptr;
-        BSN_TRY(stage_autotune(ctx, prec, pc, scratch));
-        return stage_autotune(ctx, prec, pf, scratch);
+        f64::StageArgs p[2] = {cb, fb};
+        p[0].Uin = g->Uc;
+        p[1].Uin = g->Uf; p[1].Gh = nullptr;
+        double* out[2] = {scratch, scratch + C.nelem()};
+        return stage_autotune_batch(ctx, prec, p, out, 2);
     };
     BSN_TRY(tune());
     int vc = tile_code(ctx, prec, cb);
@@ -572,6 +572,88 @@ bsn_status fmr3d_run(bsn_ctx* ctx, const bsn_fmr2* g, double cfl, int prec, int 
     bool same = S->exec && memcmp(&S->g, g, sizeof(bsn_fmr2)) == 0 && S->prec == prec && S->sg == self_gravity &&
                 S->G_grav == G_grav && S->cfl == cfl && S->t_end == t_end && S->vc == vc && S->vf == vf &&
                 memcmp(S->ptrs, ptrs, sizeof(ptrs)) == 0;
+    const int* done = &rd->done;
+    auto body = [&]() -> bsn_status {
+        BSN_TRY(f64_cfl_fold(ctx, g->Uc, g->ncx, g->ncy, g->ncz, g->dxc, g->dyc, g->dzc, g->gamma, &rd->smc,
+                             &rd->nanc));
+        BSN_TRY(f64_cfl_fold(ctx, g->Uf, g->nfx, g->nfy, g->nfz, g->dxf, g->dyf, g->dzf, g->gamma, &rd->smf,
+                             &rd->nanf));
+        run_dt_kernel<<<1, 1, 0, ctx->stream>>>(rd, cfl, r, t_end);
+        BSN_TRY(launch_check(ctx, "fmr_run_dt_kernel"));
+        if (self_gravity) {
+            BSN_TRY(fmr_poisson(ctx, g, G, phic, phif, prec != PREC_F64));
+            if (G_grav != 1.0) {
+                long long nc = (long long)g->ncx * g->ncy * g->ncz, nf = (long long)g->nfx * g->nfy * g->nfz;
+                scale_kernel<<<grid1d(nc, 256), 256, 0, ctx->stream>>>(phic, nc, G_grav);
+                BSN_TRY(launch_check(ctx, "scale_kernel"));
+                scale_kernel<<<grid1d(nf, 256), 256, 0, ctx->stream>>>(phif, nf, G_grav);
+                BSN_TRY(launch_check(ctx, "scale_kernel"));
+            }
+        }
+        int blocks;
+        grid_blocks(C.nelem(), blocks);
+        copy_kernel<<<blocks, 256, 0, ctx->stream>>>(Ucn, g->Uc, C.nelem(), done);
+        BSN_TRY(launch_check(ctx, "fmr_copy_kernel"));
+        long long nregw = (long long)(R.bytes / sizeof(double));
+        grid_blocks(nregw, blocks);
+        zero_kernel<<<blocks, 256, 0, ctx->stream>>>(R.base, nregw, done);
+        BSN_TRY(launch_check(ctx, "fmr_zero_kernel"));
+        long long nic = G.hi[0] - G.lo[0] + 1, njc = G.hi[1] - G.lo[1] + 1, nkc = G.hi[2] - G.lo[2] + 1;
+        long long nreg = 2 * 5 * (njc * nkc + nic * nkc + nic * njc);
+        const double rr = (double)(r * r);
+        // coarse step + fine subcycle 0 (ghosts from U_c^n), one launch per stage
+        BSN_TRY(prolong_ghosts(ctx, G, Ucn, nullptr, 0.0, Gh, done));
+        {
+            double* inc[3] = {g->Uc, Ac, Bc};
+            double* outc[3] = {Ac, Bc, g->Uc};
+            double* inf[3] = {g->Uf, Af, Bf};
+            double* outf[3] = {Af, Bf, g->Uf};
+            for (int s = 0; s < 3; ++s) {
+                f64::StageBatch B;
+                B.nlev = 2;
+                B.queue = &rd->queue[s];
+                B.lv[0] = cb;
+                B.lv[0].Uin = inc[s]; B.lv[0].Un = g->Uc; B.lv[0].Uout = outc[s];
+                set_stage(B.lv[0], s + 1, 0.0);
+                B.lv[0].reg.wt = rk_w[s];
+                B.lv[1] = fb;
+                B.lv[1].Uin = inf[s]; B.lv[1].Un = g->Uf; B.lv[1].Uout = outf[s];
+                set_stage(B.lv[1], s + 1, 0.0);
+                BSN_TRY(stage_launch_batch(ctx, prec, B));
+                fine_reg_kernel<<<grid1d(nreg, 128), 128, 0, ctx->stream>>>(G, R.f, 0.0, &rd->dtf, rk_w[s], rr,
+                                                                             done);
+                BSN_TRY(launch_check(ctx, "fine_reg_kernel"));
+            }
+        }
+        BSN_TRY(f64_ghost_combine(ctx, g->Uc, Bc, nullptr, g->ncx, g->ncy, g->ncz, g->bc, 0.0, &rd->dt, done));
+        BSN_TRY(f64_ghost_combine(ctx, g->Uf, nullptr, Gh, g->nfx, g->nfy, g->nfz, g->bc, 0.0, &rd->dtf, done));
+        // remaining fine subcycles: ghosts from (1-a) U_c^n + a U_c^{n+1}
+        for (int s_sub = 1; s_sub < r; ++s_sub) {
+            double alpha = (double)s_sub / (double)r;
+            BSN_TRY(prolong_ghosts(ctx, G, Ucn, g->Uc, alpha, Gh, done));
+            double* in[3] = {g->Uf, Af, Bf};
+            double* out[3] = {Af, Bf, g->Uf};
+            for (int s = 0; s < 3; ++s) {
+                f64::StageArgs a = fb;
+                a.Uin = in[s]; a.Un = g->Uf; a.Uout = out[s];
+                set_stage(a, s + 1, 0.0);
+                BSN_TRY(stage_launch(ctx, prec, a));
+                fine_reg_kernel<<<grid1d(nreg, 128), 128, 0, ctx->stream>>>(G, R.f, 0.0, &rd->dtf, rk_w[s], rr,
+                                                                             done);
+                BSN_TRY(launch_check(ctx, "fine_reg_kernel"));
+            }
+            BSN_TRY(f64_ghost_combine(ctx, g->Uf, nullptr, Gh, g->nfx, g->nfy, g->nfz, g->bc, 0.0, &rd->dtf, done));
+        }
+        // restrict, Berger-Colella correction, coarse floors, advance t
+        BSN_TRY(restrict_(ctx, G, g->Uc, g->Uf, 5, done));
+        long long ncorr = 5 * (njc * nkc + nic * nkc + nic * njc);
+        bc_correct_kernel<<<grid1d(ncorr, 128), 128, 0, ctx->stream>>>(G, R.c, R.f, g->Uc, 1.0 / g->dxc,
+                                                                        1.0 / g->dyc, 1.0 / g->dzc, done);
+        BSN_TRY(launch_check(ctx, "bc_correct_kernel"));
+        BSN_TRY(f64_floors(ctx, g->Uc, g->ncx, g->ncy, g->ncz, g->rho_floor, g->P_floor, g->gamma, done));
+        run_advance_kernel<<<1, 1, 0, ctx->stream>>>(rd);
+        return launch_check(ctx, "fmr_run_advance_kernel");
+    };
     auto capture = [&]() -> bsn_status {
         S->release();
         if (!S->cap) BSN_CUDA(ctx, cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking));
@@ -582,88 +664,6 @@ bsn_status fmr3d_run(bsn_ctx* ctx, const bsn_fmr2* g, double cfl, int prec, int 
         ctx->stream = S->cap;
         cudaError_t be = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
         if (be != cudaSuccess) { ctx->stream = user; ctx->profiling = prof; return cuda_check(ctx, be, "cudaStreamBeginCapture"); }
-        const int* done = &rd->done;
-        auto body = [&]() -> bsn_status {
-            BSN_TRY(f64_cfl_fold(ctx, g->Uc, g->ncx, g->ncy, g->ncz, g->dxc, g->dyc, g->dzc, g->gamma, &rd->smc,
-                                 &rd->nanc));
-            BSN_TRY(f64_cfl_fold(ctx, g->Uf, g->nfx, g->nfy, g->nfz, g->dxf, g->dyf, g->dzf, g->gamma, &rd->smf,
-                                 &rd->nanf));
-            run_dt_kernel<<<1, 1, 0, ctx->stream>>>(rd, cfl, r, t_end);
-            BSN_TRY(launch_check(ctx, "fmr_run_dt_kernel"));
-            if (self_gravity) {
-                BSN_TRY(fmr_poisson(ctx, g, G, phic, phif, prec != PREC_F64));
-                if (G_grav != 1.0) {
-                    long long nc = (long long)g->ncx * g->ncy * g->ncz, nf = (long long)g->nfx * g->nfy * g->nfz;
-                    scale_kernel<<<grid1d(nc, 256), 256, 0, ctx->stream>>>(phic, nc, G_grav);
-                    BSN_TRY(launch_check(ctx, "scale_kernel"));
-                    scale_kernel<<<grid1d(nf, 256), 256, 0, ctx->stream>>>(phif, nf, G_grav);
-                    BSN_TRY(launch_check(ctx, "scale_kernel"));
-                }
-            }
-            int blocks;
-            grid_blocks(C.nelem(), blocks);
-            copy_kernel<<<blocks, 256, 0, ctx->stream>>>(Ucn, g->Uc, C.nelem(), done);
-            BSN_TRY(launch_check(ctx, "fmr_copy_kernel"));
-            long long nregw = (long long)(R.bytes / sizeof(double));
-            grid_blocks(nregw, blocks);
-            zero_kernel<<<blocks, 256, 0, ctx->stream>>>(R.base, nregw, done);
-            BSN_TRY(launch_check(ctx, "fmr_zero_kernel"));
-            long long nic = G.hi[0] - G.lo[0] + 1, njc = G.hi[1] - G.lo[1] + 1, nkc = G.hi[2] - G.lo[2] + 1;
-            long long nreg = 2 * 5 * (njc * nkc + nic * nkc + nic * njc);
-            const double rr = (double)(r * r);
-            // coarse step + fine subcycle 0 (ghosts from U_c^n), one launch per stage
-            BSN_TRY(prolong_ghosts(ctx, G, Ucn, nullptr, 0.0, Gh, done));
-            {
-                double* inc[3] = {g->Uc, Ac, Bc};
-                double* outc[3] = {Ac, Bc, g->Uc};
-                double* inf[3] = {g->Uf, Af, Bf};
-                double* outf[3] = {Af, Bf, g->Uf};
-                for (int s = 0; s < 3; ++s) {
-                    f64::StageBatch B;
-                    B.nlev = 2;
-                    B.queue = &rd->queue[s];
-                    B.lv[0] = cb;
-                    B.lv[0].Uin = inc[s]; B.lv[0].Un = g->Uc; B.lv[0].Uout = outc[s];
-                    set_stage(B.lv[0], s + 1, 0.0);
-                    B.lv[0].reg.wt = rk_w[s];
-                    B.lv[1] = fb;
-                    B.lv[1].Uin = inf[s]; B.lv[1].Un = g->Uf; B.lv[1].Uout = outf[s];
-                    set_stage(B.lv[1], s + 1, 0.0);
-                    BSN_TRY(stage_launch_batch(ctx, prec, B));
-                    fine_reg_kernel<<<grid1d(nreg, 128), 128, 0, ctx->stream>>>(G, R.f, 0.0, &rd->dtf, rk_w[s], rr,
-                                                                                 done);
-                    BSN_TRY(launch_check(ctx, "fine_reg_kernel"));
-                }
-            }
-            BSN_TRY(f64_ghost_combine(ctx, g->Uc, Bc, nullptr, g->ncx, g->ncy, g->ncz, g->bc, 0.0, &rd->dt, done));
-            BSN_TRY(f64_ghost_combine(ctx, g->Uf, nullptr, Gh, g->nfx, g->nfy, g->nfz, g->bc, 0.0, &rd->dtf, done));
-            // remaining fine subcycles: ghosts from (1-a) U_c^n + a U_c^{n+1}
-            for (int s_sub = 1; s_sub < r; ++s_sub) {
-                double alpha = (double)s_sub / (double)r;
-                BSN_TRY(prolong_ghosts(ctx, G, Ucn, g->Uc, alpha, Gh, done));
-                double* in[3] = {g->Uf, Af, Bf};
-                double* out[3] = {Af, Bf, g->Uf};
-                for (int s = 0; s < 3; ++s) {
-                    f64::StageArgs a = fb;
-                    a.Uin = in[s]; a.Un = g->Uf; a.Uout = out[s];
-                    set_stage(a, s + 1, 0.0);
-                    BSN_TRY(stage_launch(ctx, prec, a));
-                    fine_reg_kernel<<<grid1d(nreg, 128), 128, 0, ctx->stream>>>(G, R.f, 0.0, &rd->dtf, rk_w[s], rr,
-                                                                                 done);
-                    BSN_TRY(launch_check(ctx, "fine_reg_kernel"));
-                }
-                BSN_TRY(f64_ghost_combine(ctx, g->Uf, nullptr, Gh, g->nfx, g->nfy, g->nfz, g->bc, 0.0, &rd->dtf, done));
-            }
-            // restrict, Berger-Colella correction, coarse floors, advance t
-            BSN_TRY(restrict_(ctx, G, g->Uc, g->Uf, 5, done));
-            long long ncorr = 5 * (njc * nkc + nic * nkc + nic * njc);
-            bc_correct_kernel<<<grid1d(ncorr, 128), 128, 0, ctx->stream>>>(G, R.c, R.f, g->Uc, 1.0 / g->dxc,
-                                                                            1.0 / g->dyc, 1.0 / g->dzc, done);
-            BSN_TRY(launch_check(ctx, "bc_correct_kernel"));
-            BSN_TRY(f64_floors(ctx, g->Uc, g->ncx, g->ncy, g->ncz, g->rho_floor, g->P_floor, g->gamma, done));
-            run_advance_kernel<<<1, 1, 0, ctx->stream>>>(rd);
-            return launch_check(ctx, "fmr_run_advance_kernel");
-        };
         bsn_status cst = body();
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
@@ -680,21 +680,25 @@ bsn_status fmr3d_run(bsn_ctx* ctx, const bsn_fmr2* g, double cfl, int prec, int 
         memcpy(S->ptrs, ptrs, sizeof(ptrs));
         return BSN_OK;
     };
-    if (!same) BSN_TRY(capture());
+    const bool direct = !same && n_steps <= kDirectSteps;
+    if (!same && !direct) BSN_TRY(capture());
     double* h = (double*)pinned(ctx, 128, &st); BSN_TRY(st);
     const bool settle = n_steps >= 2 && !tile_settled(ctx, TUNE_FMR, prec);
-    BSN_TRY(graph_replay(ctx, S->exec, S->kernels, settle ? 1 : n_steps, t_end > 0.0, &rd->done, S->ev,
-                         (volatile int*)(h + 8)));
+    auto advance = [&](int n) -> bsn_status {
+        if (direct) return launch_steps(ctx, body, n);
+        return graph_replay(ctx, S->exec, S->kernels, n, t_end > 0.0, &rd->done, S->ev,
+                         (volatile int*)(h + 8));
+    };
+    BSN_TRY(advance(settle ? 1 : n_steps));
     if (settle) {   // the tiles re-timed on the state after the first step
         BSN_TRY(tile_retime(ctx, TUNE_FMR, prec, tune));
         if (tile_code(ctx, prec, cb) != vc || tile_code(ctx, prec, fb) != vf) {
             vc = tile_code(ctx, prec, cb);
             vf = tile_code(ctx, prec, fb);
             BSN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            BSN_TRY(capture());
+            if (!direct) BSN_TRY(capture());
         }
-        BSN_TRY(graph_replay(ctx, S->exec, S->kernels, n_steps - 1, t_end > 0.0, &rd->done, S->ev,
-                             (volatile int*)(h + 8)));
+        BSN_TRY(advance(n_steps - 1));
     }
     BSN_CUDA(ctx, cudaMemcpyAsync(h, rd, sizeof(RunDev), cudaMemcpyDeviceToHost, ctx->stream));
     BSN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -365,11 +365,14 @@ bsn_status fmrN_run(bsn_ctx* ctx, const bsn_fmr2* pairs, int npairs, double cfl,
     int tiles[NMAXL] = {-1, -1, -1, -1};
     for (int l = 0; l < plan.nl; ++l) plan.base[l].tune_class = TUNE_FMR_N;
     auto tune = [&]() -> bsn_status {
+        f64::StageArgs p[NMAXL];
+        double* out[NMAXL];
         for (int l = 0; l < plan.nl; ++l) {
-            f64::StageArgs p = plan.base[l];
-            p.Uin = plan.L[l].U; p.dt_dev = nullptr; p.done_dev = nullptr; p.use_reg = 0; p.use_bnd = 0; p.Gh = nullptr;
-            BSN_TRY(stage_autotune(ctx, prec, p, plan.L[l].A));
+            p[l] = plan.base[l];
+            p[l].Uin = plan.L[l].U; p[l].Gh = nullptr;
+            out[l] = plan.L[l].A;
         }
+        BSN_TRY(stage_autotune_batch(ctx, prec, p, out, plan.nl));
         for (int l = 0; l < plan.nl; ++l) tiles[l] = tile_code(ctx, prec, plan.base[l]);
         return BSN_OK;
     };
@@ -381,6 +384,18 @@ bsn_status fmrN_run(bsn_ctx* ctx, const bsn_fmr2* pairs, int npairs, double cfl,
                 memcmp(S->key_pairs.data(), pairs, sizeof(bsn_fmr2) * npairs) == 0 && S->prec == prec &&
                 S->sg == sg && S->G_grav == G_grav && S->cfl == cfl && S->t_end == t_end &&
                 memcmp(S->tiles, tiles, sizeof(tiles)) == 0 && S->key_base == S->arena.base;
+    auto body = [&]() -> bsn_status {
+        for (int l = 0; l < plan.nl; ++l) {
+            const NLevel& v = plan.L[l];
+            BSN_TRY(f64_cfl_fold(ctx, v.U, v.nx, v.ny, v.nz, v.dx, v.dy, v.dz, plan.gamma, &plan.d->sm[l],
+                                 &plan.d->nan[l]));
+        }
+        n_dt_kernel<<<1, 1, 0, ctx->stream>>>(plan.d, cfl, plan.R, t_end, 0.0);
+        BSN_TRY(launch_check(ctx, "fmrN_dt_kernel"));
+        BSN_TRY(plan.step());
+        n_advance_kernel<<<1, 1, 0, ctx->stream>>>(plan.d);
+        return launch_check(ctx, "fmrN_advance_kernel");
+    };
     auto capture = [&]() -> bsn_status {
         S->release();
         if (!S->cap) BSN_CUDA(ctx, cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking));
@@ -391,18 +406,6 @@ bsn_status fmrN_run(bsn_ctx* ctx, const bsn_fmr2* pairs, int npairs, double cfl,
         ctx->stream = S->cap;
         cudaError_t be = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
         if (be != cudaSuccess) { ctx->stream = user; ctx->profiling = prof; return cuda_check(ctx, be, "cudaStreamBeginCapture"); }
-        auto body = [&]() -> bsn_status {
-            for (int l = 0; l < plan.nl; ++l) {
-                const NLevel& v = plan.L[l];
-                BSN_TRY(f64_cfl_fold(ctx, v.U, v.nx, v.ny, v.nz, v.dx, v.dy, v.dz, plan.gamma, &plan.d->sm[l],
-                                     &plan.d->nan[l]));
-            }
-            n_dt_kernel<<<1, 1, 0, ctx->stream>>>(plan.d, cfl, plan.R, t_end, 0.0);
-            BSN_TRY(launch_check(ctx, "fmrN_dt_kernel"));
-            BSN_TRY(plan.step());
-            n_advance_kernel<<<1, 1, 0, ctx->stream>>>(plan.d);
-            return launch_check(ctx, "fmrN_advance_kernel");
-        };
         bsn_status cst = body();
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
@@ -420,20 +423,24 @@ bsn_status fmrN_run(bsn_ctx* ctx, const bsn_fmr2* pairs, int npairs, double cfl,
         S->key_base = S->arena.base;
         return BSN_OK;
     };
-    if (!same) BSN_TRY(capture());
+    const bool direct = !same && n_steps <= kDirectSteps;
+    if (!same && !direct) BSN_TRY(capture());
     bsn_status st;
     double* h = (double*)pinned(ctx, 128 + sizeof(NDev), &st); BSN_TRY(st);
     const bool settle = n_steps >= 2 && !tile_settled(ctx, TUNE_FMR_N, prec);
-    BSN_TRY(graph_replay(ctx, S->exec, S->kernels, settle ? 1 : n_steps, t_end > 0.0, plan.done, S->ev,
-                         (volatile int*)(h + 8)));
+    auto advance = [&](int n) -> bsn_status {
+        if (direct) return launch_steps(ctx, body, n);
+        return graph_replay(ctx, S->exec, S->kernels, n, t_end > 0.0, plan.done, S->ev,
+                         (volatile int*)(h + 8));
+    };
+    BSN_TRY(advance(settle ? 1 : n_steps));
     if (settle) {   // the tiles re-timed on the state after the first step
         BSN_TRY(tile_retime(ctx, TUNE_FMR_N, prec, tune));
-        if (memcmp(S->tiles, tiles, sizeof(tiles)) != 0) {
+        if (!direct && memcmp(S->tiles, tiles, sizeof(tiles)) != 0) {
             BSN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             BSN_TRY(capture());
         }
-        BSN_TRY(graph_replay(ctx, S->exec, S->kernels, n_steps - 1, t_end > 0.0, plan.done, S->ev,
-                             (volatile int*)(h + 8)));
+        BSN_TRY(advance(n_steps - 1));
     }
     NDev* hd = (NDev*)(h + 16);
     BSN_CUDA(ctx, cudaMemcpyAsync(hd, plan.d, sizeof(NDev), cudaMemcpyDeviceToHost, ctx->stream));
