@@ -94,8 +94,10 @@ static bsn_status find_uniform(bsn_ctx* ctx, const TileVariant& v, const f64::St
     return launch_check(ctx, "uniform_tiles_kernel");
 }
 
-// Kept for uniform grids of 2^18 cells (64^3) and more with no sources: below
-// that the extra launch costs what it saves (24^3: 3 us of a 150 us step).
+// For uniform grids of 2^18 cells (64^3) and more with no sources.  Smaller
+// ones gain nothing: with and without, ms per step with a blast, FP64 / FP32:
+// 48^3 0.270 / 0.102 both ways, 64^3 0.450 / 0.172 and 0.450 / 0.177, 96^3
+// 1.03 / 0.39 and 1.25 / 0.42, 128^3 1.87 / 0.67 and 2.91 / 0.93 (B200).
 static bool uniform_tiles_apply(const f64::StageArgs& b) {
     if (b.mode != 0 || b.Gh || b.ledger || b.use_reg || b.use_bnd || b.F[0] || b.F[1] || b.F[2]) return false;
     if (b.use_bh | b.use_sg | b.use_sink | b.use_rot | b.use_damp) return false;
@@ -181,7 +183,7 @@ bsn_status stage_autotune_batch(bsn_ctx* ctx, int prec, const f64::StageArgs* pr
     }
     if (known) return BSN_OK;
     bsn_status st;
-    unsigned int* queue = (unsigned int*)slot(ctx, SLOT_RED, 64, &st);   // counter, then 4 doubles
+    unsigned int* queue = (unsigned int*)slot(ctx, SLOT_RED, 64, &st);
     BSN_TRY(st);
     f64::StageBatch B;
     B.nlev = n;
@@ -193,7 +195,6 @@ bsn_status stage_autotune_batch(bsn_ctx* ctx, int prec, const f64::StageArgs* pr
         }
         if (probes[l].tune_class == ctx->retime_class) ctx->retimed.insert(tile_key(prec, probes[l]));
         B.lv[l] = probe_args(probes[l], scratch[l]);
-        if (probes[l].ledger) B.lv[l].ledger = (double*)queue + 1;   // the ledger's kernels, into spare words
     }
     int best = 0;
     if (ctx->forced_tile[prec] >= 0) {

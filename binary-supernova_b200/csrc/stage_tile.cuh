@@ -184,7 +184,8 @@ __device__ __forceinline__ bool same_bits(double a, double b) {
 // finite.  Such a block skips its faces.  That covers the undisturbed
 // surroundings of a blast wave and gas at rest.  Measured with a blast of
 // radius 0.15-0.25 of the box at 256^3, ms per step without and with:
-// FP64 22.6 and 7.3, FP32 7.0 and 3.2, learned 9.5 and 5.2 (B200).
+// FP64 22.9 and 8.3, FP32 7.2 and 3.7, learned 10.4 and 6.0 (one-step
+// calls, the first flag pass included; B200).
 //
 // calm: the one cell's flux is certainly finite.  Its reconstructions are the
 // cell to within rounding, so with density, momentum and pressure in these
