@@ -72,7 +72,7 @@ __global__ void diag_kernel(const double* U, int nx, int ny, int nz, double dx, 
 // record {t, dt, totals} at index steps - 1 when it is below cap.  A warp per
 // total: its lanes merge every 32nd partial, then one another in a fixed tree,
 // so the result does not depend on scheduling.  (One thread per total walked
-// the partials' loads in a chain: 70 us, against 6 us.)
+// the partials' loads in a chain: 70 us, against 7 us.)
 __global__ void diag_finish(const double* part, int nblocks, double dV, double* out, const double* t,
                             const double* dt, const int* steps, const int* done, int cap, const double* ledger) {
     if (done && *done) return;

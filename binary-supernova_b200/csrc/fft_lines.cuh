@@ -300,6 +300,11 @@ struct AxisIO {
     int n_in, n_out;
 };
 
+// Bound by latency at few CTAs per SM, so the FP32 forms are register-capped
+// (4 CTAs here, 3 in z_conv_kernel); and a block takes lines on into the next
+// outer position, where one block per position had a ninth of its lanes idle
+// (n + 1 = 129 lines, 16 a block).  128^3 solve with both: FP64 187 -> 179 us,
+// FP32 115 -> 103 us.
 template <class C, int LOGN, bool INV>
 __global__ void __launch_bounds__(256, sizeof(C) == 8 ? 4 : 2) axis_kernel(AxisIO<C> io, const C* tw, int lines) {
     using Sh = LineShape<LOGN>;

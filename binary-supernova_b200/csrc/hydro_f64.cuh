@@ -49,9 +49,9 @@ bsn_status graph_replay(bsn_ctx* ctx, cudaGraphExec_t exec, int kernels, int n_s
 
 // Steps that a call on buffers without a captured graph takes as plain
 // launches: capturing and instantiating a graph costs about 180 us of host
-// time, while the launches of a step (12 to 45, some 2 us each) go on ahead of
-// the GPU.  64^3 coupled loop, 2 steps on new buffers: 1.96 ms with a graph
-// captured for them, 1.79 ms replaying one that is there.
+// time, while a step's plain launches go on ahead of the GPU.  On buffers that
+// alternate (so a graph is captured per call) against one that is there: 64^3
+// coupled loop, 2 steps, 1.94 and 1.79 ms; 64^3 run, 4 steps, 2.18 and 2.00.
 constexpr int kDirectSteps = 4;
 template <class F>
 bsn_status launch_steps(bsn_ctx* ctx, F&& body, int n_steps) {
