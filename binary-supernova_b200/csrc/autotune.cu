@@ -67,6 +67,7 @@ int tile_code(bsn_ctx* ctx, int prec, const f64::StageArgs& A) {
 }
 
 // One CTA per tile: 1 where all of its active cells hold the same words.
+// Bound by its loads, a warp per row (figures at uniform_stage_kernel).
 __global__ void uniform_tiles_kernel(const double* U, int nx, int ny, int nz, int tx, int ty, int tz,
                                      unsigned char* out) {
     const Geom G(nx, ny, nz);
@@ -76,10 +77,14 @@ __global__ void uniform_tiles_kernel(const double* U, int nx, int ny, int nz, in
     if (threadIdx.x < 5) first[threadIdx.x] = U[G.act(a0, b0, c0) + threadIdx.x];
     __syncthreads();
     bool mixed = false;
-    for (int e = threadIdx.x; e < row * rows * planes; e += blockDim.x) {
-        const int w = e % row, r = e / row;
-        const double v = U[G.act(a0, b0 + r % rows, c0 + r / rows) + w];
-        mixed |= __double_as_longlong(v) != __double_as_longlong(first[w % 5]);
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    int b = threadIdx.x >> 5, c = 0;
+    while (b >= rows) b -= rows, ++c;
+    while (c < planes) {
+        const double* u = U + G.act(a0, b0 + b, c0 + c);
+        for (int w = lane, q = lane % 5; w < row; w += 32, q = q < 3 ? q + 2 : q - 3)   // 32 words on: q + 2 mod 5
+            mixed |= __double_as_longlong(u[w]) != __double_as_longlong(first[q]);
+        for (b += warps; b >= rows; b -= rows) ++c;
     }
     const int any = __syncthreads_or(mixed);
     if (threadIdx.x == 0)

@@ -979,7 +979,9 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_list(const __grid_const
 // combined per tile; the others are listed for the stage kernel, whose CTAs
 // (registers for the faces, two or three per SM) a quiet tile would only hold.
 // Bound by its stores; 128 threads per tile and few registers keep some 2,000
-// tiles in flight.
+// tiles in flight.  A warp per row, here and in uniform_tiles_kernel, instead
+// of divisions per word: two FP32 256^3 steps 6.56 -> 6.06 ms, one FP64 step
+// 7.97 -> 7.49, two learned steps 10.9 -> 10.3.
 template <class P>
 __global__ void __launch_bounds__(128, 8) uniform_stage_kernel(const __grid_constant__ f64::StageArgs A, int tx, int ty,
                                                                 int tz) {
@@ -1030,10 +1032,13 @@ __global__ void __launch_bounds__(128, 8) uniform_stage_kernel(const __grid_cons
     const int row = 5 * min(tx, A.nx - nb[0] * tx), rows = min(ty, A.ny - nb[1] * ty),
               planes = min(tz, A.nz - nb[2] * tz);
     double* out = A.Uout + G.act(nb[0] * tx, nb[1] * ty, nb[2] * tz);
-    for (int e = tid; e < row * rows * planes; e += 128) {
-        const int i = e % row, r = e / row, q = i % 5;
-        out[i + G.sy * (r % rows) + G.sz * (r / rows)] =
-            q == 0 ? w[0] : (q == 1 ? w[1] : (q == 2 ? w[2] : (q == 3 ? w[3] : w[4])));
+    int b = tid >> 5, c = 0;   // a warp per row: no division per word
+    while (b >= rows) b -= rows, ++c;
+    while (c < planes) {
+        double* o = out + G.sy * b + G.sz * c;
+        for (int i = tid & 31, q = (tid & 31) % 5; i < row; i += 32, q = q < 3 ? q + 2 : q - 3)   // q = i mod 5
+            o[i] = q == 0 ? w[0] : (q == 1 ? w[1] : (q == 2 ? w[2] : (q == 3 ? w[3] : w[4])));
+        for (b += 4; b >= rows; b -= rows) ++c;
     }
     if (tid == 0) {
         A.uni_out[tile] = 1;
