@@ -974,8 +974,8 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_list(const __grid_const
 }
 
 // The tiles of a stage whose result is one cell: uniform in the input and the
-// base state, with the same cell in the six neighbouring tiles, calm, and no
-// sources (the host's condition).  Nothing is staged and one cell is read and
+// base state, with the same cell in the six neighbouring tiles, calm, above the
+// floors, and no sources (the host's condition).  Nothing is staged and one cell is read and
 // combined per tile; the others are listed for the stage kernel, whose CTAs
 // (registers for the faces, two or three per SM) a quiet tile would only hold.
 // Bound by its stores; 128 threads per tile and few registers keep some 2,000
@@ -1013,8 +1013,13 @@ __global__ void __launch_bounds__(128, 8) uniform_stage_kernel(const __grid_cons
 #pragma unroll
             for (int q = 0; q < 5; ++q) same = same && same_bits(A.Uin[o + q], u[q]);
         }
+        // a cell that the floors change differs from the ghosts copied from it,
+        // which stay raw: at the grid's boundary it is not uniform gas
+        const double raw[5] = {u[0], u[1], u[2], u[3], u[4]};
         typename P::real w[5], pr;
         P::stage(u, true, A, P::consts(A), w, pr);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) same = same && same_bits(u[q], raw[q]);
         w[4] = pr;
         one = __syncthreads_and(same && calm(w));
     }
