@@ -708,7 +708,7 @@ bsn_status launch_learned(bsn_ctx* ctx, const f64::StageArgs& A0) {
     }
     A.list = A.split_list;
     A.list_count = A.split_count;
-    return tile::launch_list<tile::F32Learned, TX, TY, TZ, NT, MINB>(ctx, A, smem_l, "stage_kernel_learned");
+    return tile::launch_list<tile::F32Learned, TX, TY, TZ, NT, MINB, false>(ctx, A, smem_l, "stage_kernel_learned");
 }
 }  // namespace
 

@@ -802,7 +802,9 @@ __device__ __forceinline__ bool stage_block(const f64::StageArgs& A, int a0, int
             if (!(quiet[0] && quiet[1] && quiet[2])) {
                 if (tid == 0) {
                     const int gx = (A.nx + TX - 1) / TX, gy = (A.ny + TY - 1) / TY;
-                    A.split_list[atomicAdd(A.split_count, 1u)] = a0 / TX + gx * (b0 / TY + gy * (c0 / TZ));
+                    const int t = a0 / TX + gx * (b0 / TY + gy * (c0 / TZ));
+                    A.split_list[atomicAdd(A.split_count, 1u)] = t;
+                    if (UNI) A.uni_out[t] = 0;   // its result is no more uniform than its input
                 }
                 return true;
             }
@@ -864,7 +866,7 @@ __device__ __forceinline__ bool stage_block(const f64::StageArgs& A, int a0, int
             }
         }
     }
-    if (UNI && A.uni_out) {
+    if constexpr (UNI) {
         __syncthreads();
         if (have) {
 #pragma unroll
@@ -950,8 +952,12 @@ __global__ void __launch_bounds__(NT, MINB)
 // The listed blocks of a stage (written by the launch before it on the same
 // stream), walked by a persistent grid: each CTA takes its first block by its
 // index, then draws the next from a queue counter (list_count[1], zeroed with
-// the count), so CTAs whose blocks take longer take fewer.
-template <class P, int TX, int TY, int TZ, int NT, int MINB>
+// the count), so CTAs whose blocks take longer take fewer.  UNI: the list is
+// uniform_stage_kernel's, so its tiles may still be uniform, and their results'
+// flags are kept.  A learned screen's list holds no such tile, and there the
+// test cost 5 %: a learned 256^3 step without uniform gas 32.9 ms without it
+// and 34.4 with it, 128x96x80 2.39 and 2.49.
+template <class P, int TX, int TY, int TZ, int NT, int MINB, bool UNI>
 __global__ void __launch_bounds__(NT, MINB) stage_kernel_list(const __grid_constant__ f64::StageArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ double red[NT / 32];
@@ -964,8 +970,8 @@ __global__ void __launch_bounds__(NT, MINB) stage_kernel_list(const __grid_const
     const int gx = (A.nx + TX - 1) / TX, gy = (A.ny + TY - 1) / TY;
     for (int t = blockIdx.x; t < n;) {
         const int b = A.list[t];
-        stage_block<P, TX, TY, TZ, NT, MINB, false, true>(A, (b % gx) * TX, ((b / gx) % gy) * TY, (b / (gx * gy)) * TZ, smem_raw, red,
-                                       nanflag);
+        stage_block<P, TX, TY, TZ, NT, MINB, false, UNI>(A, (b % gx) * TX, ((b / gx) % gy) * TY, (b / (gx * gy)) * TZ,
+                                                         smem_raw, red, nanflag);
         // the block's barriers order every thread's reads of `next` before this write
         if (threadIdx.x == 0) next = (int)gridDim.x + (int)atomicAdd(A.list_count + 1, 1u);
         __syncthreads();
@@ -1163,9 +1169,9 @@ bsn_status launch_plain(bsn_ctx* ctx, const f64::StageArgs& A, int smem, const c
 }
 
 // Host: the stage kernel over the blocks in A.list (a persistent grid).
-template <class P, int TX, int TY, int TZ, int NT, int MINB>
+template <class P, int TX, int TY, int TZ, int NT, int MINB, bool UNI = true>
 bsn_status launch_list(bsn_ctx* ctx, const f64::StageArgs& A, int smem, const char* name) {
-    auto fn = stage_kernel_list<P, TX, TY, TZ, NT, MINB>;
+    auto fn = stage_kernel_list<P, TX, TY, TZ, NT, MINB, UNI>;
     static int slots[64] = {0};
     const int dev = ctx->device & 63;
     if (!slots[dev]) {
