@@ -109,8 +109,9 @@ static bool uniform_tiles_apply(const f64::StageArgs& b) {
     return (long long)b.nx * b.ny * b.nz >= (1LL << 18);
 }
 
-bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int prec, const f64::StageArgs& base, UniformTiles& t) {
+bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int prec, f64::StageArgs& base, UniformTiles& t) {
     t.on = uniform_tiles_apply(base);
+    if (t.on && base.tune_class == TUNE_GENERIC) base.tune_class = TUNE_STEP;
     bsn_status st;
     if (t.on) {
         size_t tiles = 0;
@@ -283,7 +284,7 @@ bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, d
             const float find = timed([&] {
                 return find_uniform(ctx, variant(prec, v), a, a.Uin, const_cast<unsigned char*>(a.uni_in));
             });
-            if (st == BSN_OK) try_code(v | kListBit, probe.tune_class == TUNE_GENERIC ? find / 3.f : 0.f);
+            if (st == BSN_OK) try_code(v | kListBit, probe.tune_class == TUNE_STEP ? find / 3.f : 0.f);
         }
     }
     ctx->profiling = prof;

@@ -39,13 +39,18 @@ bsn_status learned_launch_batch_variant(bsn_ctx* ctx, int idx, const f64::StageB
 
 // Driver classes of StageArgs::tune_class: each keeps its own tile choices.
 enum TuneClass {
-    TUNE_GENERIC = 0,    // single stages and steps through the C ABI
+    TUNE_GENERIC = 0,    // single stages and steps through the C ABI (but TUNE_STEP's)
     TUNE_RUN = 1,        // uniform-grid device time loop (run_steps.cu)
     TUNE_COUPLED = 2,    // uniform coupled driver loop (coupled_run.cu)
     TUNE_NESTED = 3,     // nested-level coupled driver loop (coupled_run.cu)
     TUNE_FMR = 4,        // two-level FMR loop (fmr_f64.cu)
     TUNE_FMR_N = 5,      // N-level FMR loop (fmr_nlevel.cu)
     TUNE_RELAX = 6,      // relaxation loop (relax.cu)
+    // single steps that may list uniform tiles.  A right-hand side, a stage or
+    // a step with sources of the same grid cannot, and has another best tile
+    // (128^3 with a blast, FP64: a step that took a right-hand side's choice
+    // was 2.95 ms instead of 1.76)
+    TUNE_STEP = 7,
 };
 // The tile-choice code recorded for A's driver class and grid (-1: none yet).
 int tile_code(bsn_ctx* ctx, int precision, const f64::StageArgs& A);
@@ -81,8 +86,9 @@ struct UniformTiles {
         a.list_zero = count + 2 * ((s + 1) % 3);
     }
 };
-// Room for them, and the tile choice of base's grid (autotuned where it may).
-bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int precision, const f64::StageArgs& base, UniformTiles& t);
+// Room for them, and the tile choice of base's grid (autotuned where it may);
+// puts single steps into their class.
+bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int precision, f64::StageArgs& base, UniformTiles& t);
 // Those of U, for the tile choice of base's grid, and cleared counts.
 bsn_status uniform_tiles_find(bsn_ctx* ctx, int precision, const f64::StageArgs& base, const double* U,
                               const UniformTiles& t);

@@ -1,0 +1,65 @@
+"""How one context's calls bear on one another: the tile a call takes, what it
+launches and what it allocates do not depend on the calls before it."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from gpu_util import NG
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+G, DX, CFL = 5.0 / 3.0, 0.02, 0.4
+KW = dict(rho_floor=1e-6, P_floor=1e-12)
+
+
+@pytest.fixture(scope="module")
+def bsn():
+    import bsn as b
+    yield b
+    b.set_profiling(False)
+    for p in ("f64", "f32", "learned"):
+        b.set_tile(p, -1)
+
+
+def _calm(bsn, n):
+    """Uniform gas at rest around a small rough patch."""
+    U = bsn.state(*n)
+    U[0], U[4] = 1.0, 1.0 / (G - 1)
+    p = (slice(NG + 20, NG + 30),) * 3
+    r = torch.rand(10, 10, 10, generator=torch.Generator().manual_seed(3), dtype=torch.float64).cuda()
+    U[(0,) + p] += r
+    U[(4,) + p] += r
+    return U
+
+
+def _launches(bsn, names, f):
+    bsn.set_profiling(True)
+    f()
+    got = [bsn.kernel_time(k)[1] for k in names]
+    bsn.set_profiling(False)
+    return got
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("first", ["nothing", "rhs", "stage", "step"])
+def test_uniform_tiles_whatever_came_first(bsn, prec, first):
+    """A right-hand side or a stage of the same grid cannot list uniform
+    tiles; its tile choice is not the steps', nor the other way round."""
+    n, dt = (128, 128, 128), 1e-3
+    rhs, step = ((bsn.euler3d_rhs, bsn.euler3d_step) if prec == "f64"
+                 else (bsn.euler3d_rhs_f32, bsn.euler3d_step_f32))
+    U, V, F = _calm(bsn, n), bsn.state(*n), bsn.flux_arrays(*n)
+    calls = {"rhs": lambda: rhs(V, *F, U, *n, DX, DX, DX, G, **KW),
+             "stage": lambda: bsn.euler3d_stage(V, U, U, *n, DX, DX, DX, dt, G, 1, precision=prec, **KW),
+             "step": lambda: step(U, *n, DX, DX, DX, dt, G, **KW), "nothing": lambda: None}
+    bsn.set_tile(prec, -1)
+    calls[first]()
+    calls["step"]()
+    assert _launches(bsn, ["uniform_stage_kernel"], calls["step"]) == [3]
+    if first != "nothing":
+        name = "stage_kernel" if prec == "f64" else "stage_kernel_f32"
+        calls["rhs"]()
+        assert _launches(bsn, ["uniform_stage_kernel"], calls["rhs"]) == [0]
+        assert sum(_launches(bsn, [name, name + "_tma"], calls["rhs"])) == 1
