@@ -45,7 +45,7 @@ static bsn_status launch_variant(bsn_ctx* ctx, int prec, int code, const f64::St
 // wherever the context allows it
 static int forced_code(bsn_ctx* ctx, int prec, const f64::StageArgs& A) {
     const int v = ctx->forced_tile[prec] >= 0 ? ctx->forced_tile[prec] : 0;
-    return v | (ctx->tma_on ? kTmaBit : 0) | (A.uni_in ? kListBit : 0);
+    return v | (A.uni_in ? kListBit : (ctx->tma_on ? kTmaBit : 0));
 }
 static bsn_status launch_batch_variant(bsn_ctx* ctx, int prec, int idx, const f64::StageBatch& B) {
     if (prec == PREC_F64) return f64_launch_batch_variant(ctx, idx, B);

@@ -194,8 +194,9 @@ bsn_status bsn_run_steps(bsn_ctx* ctx, double* U, int nx, int ny, int nz, double
  * the grid, nx is even and no ghost buffer is involved) beside the plain
  * per-thread loader.  With on != 0 (the default) the autotuner times both
  * stagings of every tile variant and keeps the faster, and a forced variant
- * (bsn_ctx_set_tile) uses TMA wherever possible; on = 0 keeps the plain
- * loader.  Results are the same either way; the switch releases the
+ * (bsn_ctx_set_tile) uses TMA wherever possible, except in steps that keep
+ * uniform tiles (uniform grids of 2^18 cells and more without sources), where
+ * it lists the others with the plain loader; on = 0 keeps the plain loader.  Results are the same either way; the switch releases the
  * context's captured step graphs.  bsn_ctx_get_tma reports the setting,
  * bsn_ctx_get_tile_tma whether a grid's chosen tile is TMA-staged (1), not
  * (0) or not chosen yet (-1).  A staging copy that does not arrive within the

@@ -63,3 +63,19 @@ def test_uniform_tiles_whatever_came_first(bsn, prec, first):
         calls["rhs"]()
         assert _launches(bsn, ["uniform_stage_kernel"], calls["rhs"]) == [0]
         assert sum(_launches(bsn, [name, name + "_tma"], calls["rhs"])) == 1
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_reported_staging_is_the_one_that_runs(bsn, prec):
+    n = (64, 64, 64)
+    step = bsn.euler3d_step if prec == "f64" else bsn.euler3d_step_f32
+    name = "stage_kernel_tma" if prec == "f64" else "stage_kernel_f32_tma"
+    U = _calm(bsn, n)
+    for tma in (True, False):
+        bsn.set_tma(tma)
+        for v in range(bsn.tile_variants(prec)):
+            bsn.set_tile(prec, v)
+            k, = _launches(bsn, [name], lambda: step(U, *n, DX, DX, DX, 1e-3, G, **KW))
+            assert bsn.get_tile_tma(*n, prec) == (k > 0), (tma, v, k)
+    bsn.set_tma(True)
+    bsn.set_tile(prec, -1)
