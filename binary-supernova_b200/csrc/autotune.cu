@@ -113,6 +113,13 @@ bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int prec, f64::StageArgs& base, U
     t.on = uniform_tiles_apply(base);
     if (t.on && base.tune_class == TUNE_GENERIC) base.tune_class = TUNE_STEP;
     bsn_status st;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(ctx->stream, &cs);
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
+    if (capturing) {   // no timing and no allocation in a capture: an earlier choice and its room, or none
+        const int code = tile_code(ctx, prec, base);
+        t.on = t.on && code >= 0 && (code & kListBit);
+    }
     if (t.on) {
         size_t tiles = 0;
         for (int v = 0; v < variant_count(prec); ++v) {
@@ -121,19 +128,18 @@ bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int prec, f64::StageArgs& base, U
                                         ((base.nz + q.tz - 1) / q.tz));
         }
         tiles = (tiles + 255) / 256 * 256;
-        unsigned char* f = (unsigned char*)slot(ctx, SLOT_UNIFORM, 256 + (3 + sizeof(int)) * tiles, &st);
+        const size_t bytes = 256 + (3 + sizeof(int)) * tiles;
+        if (capturing && ctx->slot_bytes[SLOT_UNIFORM] < bytes) {
+            t.on = false;
+            return BSN_OK;
+        }
+        unsigned char* f = (unsigned char*)slot(ctx, SLOT_UNIFORM, bytes, &st);
         BSN_TRY(st);
         t.count = (unsigned int*)f;
         t.list = (int*)(f + 256);
         for (int i = 0; i < 3; ++i) t.f[i] = f + 256 + (sizeof(int) + i) * tiles;
     }
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(ctx->stream, &cs);
-    if (cs != cudaStreamCaptureStatusNone) {   // no timing during a capture: an earlier choice, or none
-        const int code = tile_code(ctx, prec, base);
-        t.on = t.on && code >= 0 && (code & kListBit);
-        return BSN_OK;
-    }
+    if (capturing) return BSN_OK;
     f64::StageArgs p = base;
     t.set(p, 0);
     double* scratch = nullptr;

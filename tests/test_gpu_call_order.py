@@ -79,3 +79,37 @@ def test_reported_staging_is_the_one_that_runs(bsn, prec):
             assert bsn.get_tile_tma(*n, prec) == (k > 0), (tma, v, k)
     bsn.set_tma(True)
     bsn.set_tile(prec, -1)
+
+
+def test_step_captured_on_a_grid_not_seen_before(bsn):
+    """A program that captures a step after another call has sized the
+    workspace (a longer, thinner grid, too small for uniform tiles): the
+    capture neither times tiles nor allocates."""
+    from bsn._lib import load
+    L = load()
+    n, warm, dt = (64, 64, 64), (16, 16, 1000), 1e-3
+    U = _calm(bsn, n)
+    ref = U.clone()
+    bsn.euler3d_step(ref, *n, DX, DX, DX, dt, G, **KW)
+    W = bsn.state(*warm)
+    W[0], W[4] = 1.0, 1.0 / (G - 1)
+    s, ctx = torch.cuda.Stream(), C.c_void_p()
+    torch.cuda.synchronize()
+    assert L.bsn_ctx_create(C.byref(ctx), 0, C.c_void_p(s.cuda_stream)) == 0
+    try:
+        def step(A, m):
+            return L.bsn_euler3d_step_f64(ctx, C.c_void_p(A.data_ptr()), *m, DX, DX, DX, dt, G, 0, KW["rho_floor"],
+                                          KW["P_floor"])
+        assert step(W, warm) == 0
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            rc = step(U, n)
+        assert rc == 0, L.bsn_last_error(ctx).decode()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(U, ref)
+        del g
+    finally:
+        torch.cuda.synchronize()
+        L.bsn_ctx_destroy(ctx)
