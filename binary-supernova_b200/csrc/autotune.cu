@@ -128,7 +128,12 @@ bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int prec, f64::StageArgs& base, U
                                         ((base.nz + q.tz - 1) / q.tz));
         }
         tiles = (tiles + 255) / 256 * 256;
-        const size_t bytes = 256 + (3 + sizeof(int)) * tiles;
+        // Room for every grid that the stage buffers have room for (per axis at
+        // most 1/7 tile per stored cell of n + 6 for the longer tile edges, 1/4
+        // for the shortest): it moves when they do, so a step that the caller
+        // captured stays as valid as its stage buffers.
+        const size_t most = ctx->slot_bytes[SLOT_A] / (5 * sizeof(double)) / 196 + 256;
+        const size_t bytes = 256 + (3 + sizeof(int)) * std::max(tiles, most / 256 * 256 + 256);
         if (capturing && ctx->slot_bytes[SLOT_UNIFORM] < bytes) {
             t.on = false;
             return BSN_OK;

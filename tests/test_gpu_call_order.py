@@ -113,3 +113,44 @@ def test_step_captured_on_a_grid_not_seen_before(bsn):
     finally:
         torch.cuda.synchronize()
         L.bsn_ctx_destroy(ctx)
+
+
+def test_captured_step_outlives_a_step_on_another_grid(bsn):
+    """A captured step holds the workspace's addresses: a later step on a grid
+    with more tiles, which the stage buffers have room for, moves none of it."""
+    from bsn._lib import load
+    L = load()
+    dt = 1e-3
+    n, other, room = (64, 64, 64), (72, 72, 72), (16, 16, 1000)
+    U, V, W = _calm(bsn, n), _calm(bsn, other), bsn.state(*room)
+    W[0], W[4] = 1.0, 1.0 / (G - 1)
+    ref = U.clone()
+    for _ in range(2):
+        bsn.euler3d_step(ref, *n, DX, DX, DX, dt, G, **KW)
+    s, ctx = torch.cuda.Stream(), C.c_void_p()
+    torch.cuda.synchronize()
+    assert L.bsn_ctx_create(C.byref(ctx), 0, C.c_void_p(s.cuda_stream)) == 0
+    try:
+        def step(A, m):
+            rc = L.bsn_euler3d_step_f64(ctx, C.c_void_p(A.data_ptr()), *m, DX, DX, DX, dt, G, 0, KW["rho_floor"],
+                                        KW["P_floor"])
+            assert rc == 0, L.bsn_last_error(ctx).decode()
+        assert L.bsn_ctx_set_tile(ctx, 0, 1) == 0     # forced: lists the tiles that are not uniform
+        step(W, room)
+        step(U, n)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            step(U, n)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        step(V, other)
+        torch.cuda.synchronize()
+        assert torch.cuda.mem_get_info()[0] == free
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(U, ref)
+        del g
+    finally:
+        torch.cuda.synchronize()
+        L.bsn_ctx_destroy(ctx)
