@@ -300,13 +300,27 @@ struct AxisIO {
     int n_in, n_out;
 };
 
-// Bound by latency at few CTAs per SM, so the FP32 forms are register-capped
-// (4 CTAs here, 3 in z_conv_kernel); and a block takes lines on into the next
-// outer position, where one block per position had a ninth of its lanes idle
-// (n + 1 = 129 lines, 16 a block).  128^3 solve with both: FP64 187 -> 179 us,
-// FP32 115 -> 103 us.
+// CTAs per SM that the FP32 forms' registers are capped for.  The passes are
+// bound by latency at few CTAs per SM, but a cap spills, and how much depends on
+// the line's length: measured for each, us of the y passes and of the z pass
+// without a cap and with 4 (y) or 3 (z), B200:
+//   256 points (128^3)        35.7, 32.7    39.4, 37.3
+//   512 (256^3)               276, 255      414, 517    432 B spilled in z
+//   512 (64x256x32's y)       21.4, 25.5                21.4 with 3
+//   1024 (512^3)              2657, 2553    5046, 4949
+//   64 (64x256x32's z)                      12.8, 14.9
+//   128 (256x256x64's z)                    66.1, 59.9
+// Longer lines are not measured and not capped.
+template <class C, int LOGN>
+constexpr int axis_ctas() { return sizeof(C) != 8 || LOGN > 10 ? 2 : (LOGN == 9 ? 3 : 4); }
+template <class C, int LOGN>
+constexpr int conv_ctas() { return sizeof(C) == 8 && (LOGN == 7 || LOGN == 8 || LOGN == 10) ? 3 : 2; }
+
+// A block takes lines on into the next outer position, where one block per
+// position had a ninth of its lanes idle (n + 1 = 129 lines, 16 a block).
+// 128^3 solve with that and the caps: FP64 187 -> 179 us, FP32 115 -> 103 us.
 template <class C, int LOGN, bool INV>
-__global__ void __launch_bounds__(256, sizeof(C) == 8 ? 4 : 2) axis_kernel(AxisIO<C> io, const C* tw, int lines) {
+__global__ void __launch_bounds__(256, axis_ctas<C, LOGN>()) axis_kernel(AxisIO<C> io, const C* tw, int lines) {
     using Sh = LineShape<LOGN>;
     using R = typename Cx<C>::R;
     constexpr int E = Sh::E, T = Sh::T;
@@ -339,7 +353,7 @@ __global__ void __launch_bounds__(256, sizeof(C) == 8 ? 4 : 2) axis_kernel(AxisI
 // ky0 = 0, nky = N2 on one GPU; a rank's share of it after the transpose of
 // a z-slab decomposition), z < nz in and out.
 template <class C, int LOGN>
-__global__ void __launch_bounds__(256, sizeof(C) == 8 ? 3 : 2) z_conv_kernel(C* W2, const typename Cx<C>::R* khat, int nx, int N2, int ny,
+__global__ void __launch_bounds__(256, conv_ctas<C, LOGN>()) z_conv_kernel(C* W2, const typename Cx<C>::R* khat, int nx, int N2, int ny,
                                                      int nz, int lines, const C* tw, int ky0, int nky) {
     using Sh = LineShape<LOGN>;
     using R = typename Cx<C>::R;
