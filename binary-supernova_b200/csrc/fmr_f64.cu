@@ -550,13 +550,10 @@ bsn_status fmr3d_run(bsn_ctx* ctx, const bsn_fmr2* g, double cfl, int prec, int 
 
     // tile choices before any capture (the autotuner launches and times)
     auto tune = [&]() -> bsn_status {
-        bsn_status ts;
-        double* scratch = (double*)slot(ctx, SLOT_UN, sizeof(double) * (C.nelem() + F.nelem()), &ts);
-        BSN_TRY(ts);
         f64::StageArgs p[2] = {cb, fb};
         p[0].Uin = g->Uc;
         p[1].Uin = g->Uf; p[1].Gh = nullptr;
-        double* out[2] = {scratch, scratch + C.nelem()};
+        double* out[2] = {Ac, Af};   // where the first stages write
         return stage_autotune_batch(ctx, prec, p, out, 2);
     };
     BSN_TRY(tune());

@@ -154,3 +154,29 @@ def test_captured_step_outlives_a_step_on_another_grid(bsn):
     finally:
         torch.cuda.synchronize()
         L.bsn_ctx_destroy(ctx)
+
+
+def test_two_level_loop_takes_no_more_memory_than_its_levels(bsn):
+    """The loop's workspace: two stage buffers a level, the coarse state before
+    the step, the fine ghosts, and the registers of the coarse-fine faces; the
+    tile choice is timed in them."""
+    from bsn._lib import load
+    L = load()
+    m = 128
+    U = _calm(bsn, (m, m, m))
+    H = bsn.FMRGrid3D(U, m, m, m, DX, 33, 96, 33, 96, 33, 96, 2, G, **KW)
+    bsn.fmr3d_run_steps(H, CFL, n_steps=1)     # loads the kernels
+    ctx = C.c_void_p()
+    torch.cuda.synchronize()
+    assert L.bsn_ctx_create(C.byref(ctx), 0, C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    try:
+        t, k = C.c_double(0.0), C.c_int(0)
+        free = torch.cuda.mem_get_info()[0]
+        assert L.bsn_fmr3d_run_steps(ctx, C.byref(H.s), CFL, 1, 0, 1.0, 1, 0.0, C.byref(t), C.byref(k)) == 0
+        torch.cuda.synchronize()
+        state, faces = 5 * 8 * (m + 6) ** 3, 5 * 8 * 6 * m * m
+        # allocations are rounded up to 2 MiB each; well under one more state
+        assert free - torch.cuda.mem_get_info()[0] < 6 * state + 4 * faces + 8 * (2 << 20)
+    finally:
+        torch.cuda.synchronize()
+        L.bsn_ctx_destroy(ctx)
