@@ -257,13 +257,7 @@ struct State {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int kernels = 0;
-    // key of the captured graph
-    double* U = nullptr;
-    int nx = 0, ny = 0, nz = 0, nbh = -1, prec = -1, variant = -1, sg = 0, torque_free = 0, evolve = 0;
-    double dx = 0, x0 = 0, y0 = 0, z0 = 0, gamma = 0, cfl = 0, dt_max = 0, f_sink = 0, rho_floor = 0, P_floor = 0,
-           t_on = 0, rho_min = 0, t_end = 0;
-    const void* ptrs[7] = {};
-    int diag_cap = 0;
+    std::string key, last;   // of the captured step, of the last call
     cudaStream_t cap = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     void release() {
@@ -369,13 +363,13 @@ extern "C" bsn_status bsn_coupled_run_steps(bsn_ctx* ctx, double* U, bsn_bh* bhs
     if (!ctx->coupled_run_state) ctx->coupled_run_state = new State();
     State* S = (State*)ctx->coupled_run_state;
     const void* ptrs[7] = {A, B, r, part, phi, diag_out, dpart};
-    bool same = S->exec && S->U == U && S->nx == nx && S->ny == ny && S->nz == nz && S->nbh == nbh &&
-                S->prec == precision && S->variant == variant && S->sg == self_gravity &&
-                S->torque_free == torque_free && S->evolve == evolve_orbit && S->dx == dx && S->x0 == x0 &&
-                S->y0 == y0 && S->z0 == z0 && S->gamma == gamma && S->cfl == cfl && S->dt_max == dt_max &&
-                S->f_sink == f_sink && S->rho_floor == rho_floor && S->P_floor == P_floor &&
-                S->t_on == t_bh2_sink_on && S->rho_min == rho_sink_min && S->t_end == t_end &&
-                S->diag_cap == diag_cap && memcmp(S->ptrs, ptrs, sizeof(ptrs)) == 0;
+    auto key = [&] {
+        return graph_key(U, nx, ny, nz, nbh, precision, variant, self_gravity, torque_free, evolve_orbit, dx, x0, y0,
+                         z0, gamma, cfl, dt_max, f_sink, rho_floor, P_floor, t_bh2_sink_on, rho_sink_min, t_end,
+                         diag_cap, ptrs);
+    };
+    const std::string now = key();
+    const bool same = S->exec && S->key == now;
     auto body = [&]() -> bsn_status {
         dt_kernel<<<1, 1, 0, ctx->stream>>>(r, cfl, t_end, dt_max);
         BSN_TRY(launch_check(ctx, "coupled_dt_kernel"));
@@ -448,16 +442,11 @@ extern "C" bsn_status bsn_coupled_run_steps(bsn_ctx* ctx, double* U, bsn_bh* bhs
         BSN_CUDA(ctx, e);
         S->graph = graph;
         BSN_CUDA(ctx, cudaGraphInstantiate(&S->exec, graph, 0));
-        S->U = U; S->nx = nx; S->ny = ny; S->nz = nz; S->nbh = nbh; S->prec = precision; S->variant = variant;
-        S->sg = self_gravity; S->torque_free = torque_free; S->evolve = evolve_orbit; S->dx = dx; S->x0 = x0;
-        S->y0 = y0; S->z0 = z0; S->gamma = gamma; S->cfl = cfl; S->dt_max = dt_max; S->f_sink = f_sink;
-        S->rho_floor = rho_floor; S->P_floor = P_floor; S->t_on = t_bh2_sink_on; S->rho_min = rho_sink_min;
-        S->t_end = t_end;
-        S->diag_cap = diag_cap;
-        memcpy(S->ptrs, ptrs, sizeof(ptrs));
+        S->key = key();
         return BSN_OK;
     };
-    const bool direct = !same && n_steps <= kDirectSteps;
+    const bool direct = !same && n_steps <= kDirectMany && S->last != now;
+    S->last = now;
     if (!same && !direct) BSN_TRY(capture());
     const bool settle = n_steps >= 2 && !tile_settled(ctx, TUNE_COUPLED, precision);
     auto advance = [&](int n) -> bsn_status {
@@ -603,14 +592,14 @@ extern "C" bsn_status bsn_coupled_nested_run_steps(bsn_ctx* ctx, const bsn_fmr2*
     BSN_TRY(tune());
 
     const NLevel& fin = plan.L[nl - 1];
-    std::vector<double> extra = {(double)nbh, x0, y0, z0, dt_max, f_sink, (double)torque_free, t_bh2_sink_on,
-                                 rho_sink_min, (double)evolve_orbit, (double)diag_cap,
-                                 (double)(uintptr_t)r, (double)(uintptr_t)part, (double)(uintptr_t)diag_out,
-                                 (double)(uintptr_t)dpart};
-    bool same = S->exec && (int)S->key_pairs.size() == npairs &&
-                memcmp(S->key_pairs.data(), pairs, sizeof(bsn_fmr2) * npairs) == 0 && S->prec == precision &&
-                S->sg == self_gravity && S->cfl == cfl && S->t_end == t_end &&
-                memcmp(S->tiles, tiles, sizeof(tiles)) == 0 && S->key_base == S->arena.base && S->key_extra == extra;
+    auto key = [&] {
+        return graph_key(npairs, precision, self_gravity, cfl, t_end, tiles, S->arena.base, nbh, x0, y0, z0, dt_max,
+                         f_sink, torque_free, t_bh2_sink_on, rho_sink_min, evolve_orbit, diag_cap, r, part, diag_out,
+                         dpart) +
+               std::string((const char*)pairs, sizeof(bsn_fmr2) * npairs);
+    };
+    const std::string now = key();
+    const bool same = S->exec && S->key == now;
     auto body = [&]() -> bsn_status {
         for (int l = 0; l < nl; ++l) {
             const NLevel& v = plan.L[l];
@@ -684,14 +673,11 @@ extern "C" bsn_status bsn_coupled_nested_run_steps(bsn_ctx* ctx, const bsn_fmr2*
         BSN_CUDA(ctx, e);
         S->graph = graph;
         BSN_CUDA(ctx, cudaGraphInstantiate(&S->exec, graph, 0));
-        S->key_pairs.assign(pairs, pairs + npairs);
-        S->prec = precision; S->sg = self_gravity; S->G_grav = 1.0; S->cfl = cfl; S->t_end = t_end;
-        memcpy(S->tiles, tiles, sizeof(tiles));
-        S->key_base = S->arena.base;
-        S->key_extra = extra;
+        S->key = key();
         return BSN_OK;
     };
-    const bool direct = !same && n_steps <= kDirectSteps;
+    const bool direct = !same && n_steps <= kDirectMany && S->last != now;
+    S->last = now;
     if (!same && !direct) BSN_TRY(capture());
     const bool settle = n_steps >= 2 && !tile_settled(ctx, TUNE_NESTED, precision);
     auto advance = [&](int n) -> bsn_status {
@@ -702,7 +688,7 @@ extern "C" bsn_status bsn_coupled_nested_run_steps(bsn_ctx* ctx, const bsn_fmr2*
     BSN_TRY(advance(settle ? 1 : n_steps));
     if (settle) {   // the tiles re-timed on the state after the first step
         BSN_TRY(tile_retime(ctx, TUNE_NESTED, precision, tune));
-        if (!direct && memcmp(S->tiles, tiles, sizeof(tiles)) != 0) {
+        if (!direct && S->key != key()) {
             BSN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             BSN_TRY(capture());
         }

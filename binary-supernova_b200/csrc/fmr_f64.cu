@@ -475,11 +475,7 @@ struct RunState {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int kernels = 0;
-    // key of the captured graph
-    bsn_fmr2 g;
-    int prec = -1, sg = 0, vc = -1, vf = -1;
-    double G_grav = 0, cfl = 0, t_end = 0;
-    const void* ptrs[12] = {};
+    std::string key, last;   // of the captured step, of the last call
     cudaStream_t cap = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     void release() {
@@ -566,9 +562,9 @@ bsn_status fmr3d_run(bsn_ctx* ctx, const bsn_fmr2* g, double cfl, int prec, int 
     if (!ctx->fmr_run_state) ctx->fmr_run_state = new RunState();
     RunState* S = (RunState*)ctx->fmr_run_state;
     const void* ptrs[12] = {Ucn, Ac, Bc, Gh, Af, Bf, rd, R.base, R.f.bnd[0], phic, phif, nullptr};
-    bool same = S->exec && memcmp(&S->g, g, sizeof(bsn_fmr2)) == 0 && S->prec == prec && S->sg == self_gravity &&
-                S->G_grav == G_grav && S->cfl == cfl && S->t_end == t_end && S->vc == vc && S->vf == vf &&
-                memcmp(S->ptrs, ptrs, sizeof(ptrs)) == 0;
+    auto key = [&] { return graph_key(*g, prec, self_gravity, G_grav, cfl, t_end, vc, vf, ptrs); };
+    const std::string now = key();
+    const bool same = S->exec && S->key == now;
     const int* done = &rd->done;
     auto body = [&]() -> bsn_status {
         BSN_TRY(f64_cfl_fold(ctx, g->Uc, g->ncx, g->ncy, g->ncz, g->dxc, g->dyc, g->dzc, g->gamma, &rd->smc,
@@ -672,12 +668,11 @@ bsn_status fmr3d_run(bsn_ctx* ctx, const bsn_fmr2* g, double cfl, int prec, int 
         BSN_CUDA(ctx, e);
         S->graph = graph;
         BSN_CUDA(ctx, cudaGraphInstantiate(&S->exec, graph, 0));
-        S->g = *g; S->prec = prec; S->sg = self_gravity; S->G_grav = G_grav; S->cfl = cfl; S->t_end = t_end;
-        S->vc = vc; S->vf = vf;
-        memcpy(S->ptrs, ptrs, sizeof(ptrs));
+        S->key = key();
         return BSN_OK;
     };
-    const bool direct = !same && n_steps <= kDirectSteps;
+    const bool direct = !same && n_steps <= kDirectMany && S->last != now;
+    S->last = now;
     if (!same && !direct) BSN_TRY(capture());
     double* h = (double*)pinned(ctx, 128, &st); BSN_TRY(st);
     const bool settle = n_steps >= 2 && !tile_settled(ctx, TUNE_FMR, prec);

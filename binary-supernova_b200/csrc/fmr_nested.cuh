@@ -52,12 +52,7 @@ struct NState {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int kernels = 0;
-    std::vector<bsn_fmr2> key_pairs;
-    int prec = -1, sg = 0;
-    double G_grav = 0, cfl = 0, t_end = 0;
-    int tiles[NMAXL] = {-1, -1, -1, -1};
-    void* key_base = nullptr;
-    std::vector<double> key_extra;   // further parameters of the captured step (coupled loop)
+    std::string key, last;   // of the captured step, of the last call
     cudaStream_t cap = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     void release() {

@@ -380,10 +380,12 @@ bsn_status fmrN_run(bsn_ctx* ctx, const bsn_fmr2* pairs, int npairs, double cfl,
     n_init_kernel<<<1, 1, 0, ctx->stream>>>(plan.d, *t_inout);
     BSN_TRY(launch_check(ctx, "fmrN_init_kernel"));
 
-    bool same = S->exec && (int)S->key_pairs.size() == npairs &&
-                memcmp(S->key_pairs.data(), pairs, sizeof(bsn_fmr2) * npairs) == 0 && S->prec == prec &&
-                S->sg == sg && S->G_grav == G_grav && S->cfl == cfl && S->t_end == t_end &&
-                memcmp(S->tiles, tiles, sizeof(tiles)) == 0 && S->key_base == S->arena.base;
+    auto key = [&] {
+        return graph_key(npairs, prec, sg, G_grav, cfl, t_end, tiles, S->arena.base) +
+               std::string((const char*)pairs, sizeof(bsn_fmr2) * npairs);
+    };
+    const std::string now = key();
+    const bool same = S->exec && S->key == now;
     auto body = [&]() -> bsn_status {
         for (int l = 0; l < plan.nl; ++l) {
             const NLevel& v = plan.L[l];
@@ -417,13 +419,11 @@ bsn_status fmrN_run(bsn_ctx* ctx, const bsn_fmr2* pairs, int npairs, double cfl,
         BSN_CUDA(ctx, e);
         S->graph = graph;
         BSN_CUDA(ctx, cudaGraphInstantiate(&S->exec, graph, 0));
-        S->key_pairs.assign(pairs, pairs + npairs);
-        S->prec = prec; S->sg = sg; S->G_grav = G_grav; S->cfl = cfl; S->t_end = t_end;
-        memcpy(S->tiles, tiles, sizeof(tiles));
-        S->key_base = S->arena.base;
+        S->key = key();
         return BSN_OK;
     };
-    const bool direct = !same && n_steps <= kDirectSteps;
+    const bool direct = !same && n_steps <= kDirectMany && S->last != now;
+    S->last = now;
     if (!same && !direct) BSN_TRY(capture());
     bsn_status st;
     double* h = (double*)pinned(ctx, 128 + sizeof(NDev), &st); BSN_TRY(st);
@@ -436,7 +436,7 @@ bsn_status fmrN_run(bsn_ctx* ctx, const bsn_fmr2* pairs, int npairs, double cfl,
     BSN_TRY(advance(settle ? 1 : n_steps));
     if (settle) {   // the tiles re-timed on the state after the first step
         BSN_TRY(tile_retime(ctx, TUNE_FMR_N, prec, tune));
-        if (!direct && memcmp(S->tiles, tiles, sizeof(tiles)) != 0) {
+        if (!direct && S->key != key()) {
             BSN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             BSN_TRY(capture());
         }

@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstring>
 #include <algorithm>
+#include <string>
 
 #include "stage_f64.cuh"
 
@@ -47,12 +48,29 @@ bsn_status cfl_from_device(bsn_ctx* ctx, const unsigned long long* red, double c
 bsn_status graph_replay(bsn_ctx* ctx, cudaGraphExec_t exec, int kernels, int n_steps, bool until_done,
                         const int* done_dev, cudaEvent_t ev[2], volatile int* hflag);
 
-// Steps that a call on buffers without a captured graph takes as plain
-// launches: capturing and instantiating a graph costs about 180 us of host
-// time, while a step's plain launches go on ahead of the GPU.  On buffers that
-// alternate (so a graph is captured per call) against one that is there: 64^3
-// coupled loop, 2 steps, 1.94 and 1.79 ms; 64^3 run, 4 steps, 2.18 and 2.00.
-constexpr int kDirectSteps = 4;
+// Steps that a first call takes as plain launches instead of capturing a
+// graph.  A capture costs host time (130 us for the uniform loop, 190 for the
+// coupled and two-level loops, 400 for three nested levels), and every step of
+// plain launches leaves longer gaps between its kernels, so few steps are
+// cheaper without and many with one.  Calls on two buffers in turn, captured
+// and direct, us (B200): uniform loop, FP32 48^3, 1 / 4 / 8 / 12 steps, 267 /
+// 522 / 857 / 1182 and 133 / 406 / 770 / 1131, 128^3 4 / 6 steps 2804 / 4145
+// and 2819 / 4179; coupled 64^3 FP64 2 / 4 / 6 steps 1705 / 3049 / 4415 and
+// 1582 / 3038 / 4494, 128^3 FP32 1 / 2 / 3 steps 2495 / 4758 / 7045 and 2450 /
+// 4772 / 7110; two levels 32^3 2 / 3 / 4 steps 924 / 1248 / 1573 and 828 / 1220
+// / 1600; three nested levels of the binary 64^3 1 / 2 / 3 steps 3306 / 6312 /
+// 9378 and 3114 / 6314 / 9597.  A second call in a row with the same key
+// (graph_key) captures whatever its steps: a program that advances one state
+// by a step or two per call replays its graph from the third call on.
+constexpr int kDirectUniform = 4;   // the uniform loop: some ten kernels a step
+constexpr int kDirectMany = 2;      // the other loops: 40 to 120
+// What a captured step holds, as bytes: the same bytes, the same step.
+template <class... T>
+std::string graph_key(const T&... v) {
+    std::string k;
+    (k.append((const char*)&v, sizeof(v)), ...);
+    return k;
+}
 template <class F>
 bsn_status launch_steps(bsn_ctx* ctx, F&& body, int n_steps) {
     const bool prof = ctx->profiling;   // as the graphs, outside the per-kernel records

@@ -56,13 +56,7 @@ struct State {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int kernels = 0;
-    // key of the captured graph
-    double* U = nullptr;
-    int nx = 0, ny = 0, nz = 0, bc = 0, prec = 0, variant = -1;
-    double dx = 0, dy = 0, dz = 0, gamma = 0, cfl = 0, rho_floor = 0, P_floor = 0, t_end = 0;
-    double *A = nullptr, *B = nullptr;
-    const unsigned char* uni = nullptr;
-    Dev* r = nullptr;
+    std::string key, last;   // of the captured step, of the last call
     cudaStream_t cap = nullptr;   // private stream used only to capture (the caller's may be the legacy stream)
     cudaEvent_t flag_ev[2] = {nullptr, nullptr};   // done-flag readbacks of the replay chunks
 };
@@ -239,10 +233,13 @@ extern "C" bsn_status bsn_run_steps(bsn_ctx* ctx, double* U, int nx, int ny, int
     BSN_TRY(launch_check(ctx, "run_init_kernel"));
     BSN_TRY(f64_cfl_fold(ctx, U, nx, ny, nz, dx, dy, dz, gamma, &r->smax, &r->nanflag));
 
-    bool same = S->exec && S->U == U && S->nx == nx && S->ny == ny && S->nz == nz && S->dx == dx && S->dy == dy &&
-                S->dz == dz && S->gamma == gamma && S->cfl == cfl && S->bc == bc && S->rho_floor == rho_floor &&
-                S->P_floor == P_floor && S->prec == precision && S->t_end == t_end && S->variant == variant &&
-                S->A == A && S->B == B && S->r == r && S->uni == (uni.on ? uni.f[0] : nullptr);
+    auto key = [&] {
+        const unsigned char* flags = uni.on ? uni.f[0] : nullptr;
+        return graph_key(U, nx, ny, nz, dx, dy, dz, gamma, cfl, bc, rho_floor, P_floor, precision, t_end, variant, A,
+                         B, r, flags);
+    };
+    const std::string now = key();
+    const bool same = S->exec && S->key == now;
     auto body = [&]() -> bsn_status {   // one step
         dt_kernel<<<1, 1, 0, ctx->stream>>>(r, cfl, t_end);
         BSN_TRY(launch_check(ctx, "run_dt_kernel"));
@@ -286,13 +283,11 @@ extern "C" bsn_status bsn_run_steps(bsn_ctx* ctx, double* U, int nx, int ny, int
         BSN_CUDA(ctx, e);
         S->graph = g;
         BSN_CUDA(ctx, cudaGraphInstantiate(&S->exec, g, 0));
-        S->U = U; S->nx = nx; S->ny = ny; S->nz = nz; S->dx = dx; S->dy = dy; S->dz = dz; S->gamma = gamma;
-        S->cfl = cfl; S->bc = bc; S->rho_floor = rho_floor; S->P_floor = P_floor; S->prec = precision;
-        S->t_end = t_end; S->variant = variant; S->A = A; S->B = B; S->r = r;
-        S->uni = uni.on ? uni.f[0] : nullptr;
+        S->key = key();
         return BSN_OK;
     };
-    const bool direct = !same && n_steps <= kDirectSteps;
+    const bool direct = !same && n_steps <= kDirectUniform && S->last != now;
+    S->last = now;
     if (!same && !direct) BSN_TRY(capture());
     double* h = (double*)pinned(ctx, 128, &st); BSN_TRY(st);
     // replays after t_end are no-ops: with t_end, stop once the device says done

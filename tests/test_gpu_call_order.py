@@ -180,3 +180,62 @@ def test_two_level_loop_takes_no_more_memory_than_its_levels(bsn):
     finally:
         torch.cuda.synchronize()
         L.bsn_ctx_destroy(ctx)
+
+
+def _loops(bsn, prec):
+    """The device loops on a small grid: {name: (state tensors, advance by n
+    steps from time t -> (t, steps))}."""
+    m, out = 16, {}
+    gen = torch.Generator().manual_seed(5)
+
+    def gas(k):
+        U = bsn.state(k, k, k)
+        U[0] = 1.0 + 0.2 * torch.rand(U.shape[1:], generator=gen, dtype=torch.float64).cuda()
+        U[4] = 2.0 * U[0]
+        return U
+    U = gas(m)
+    out["run"] = ([U], lambda n, t: bsn.run_steps(U, m, m, m, DX, DX, DX, G, CFL, n_steps=n, t=t, precision=prec, **KW))
+    V = gas(m)
+    bhs = [bsn.BlackHole((0.05, 0.0, 0.0), (0.0, 0.3, 0.0), 0.1, 2 * DX, 1e6, 4 * DX)]
+    out["coupled"] = ([V], lambda n, t: bsn.coupled_run_steps(V, bhs, m, m, m, DX, -8 * DX, -8 * DX, -8 * DX, G, CFL,
+                                                              n_steps=n, t=t, self_gravity=True, precision=prec, **KW))
+    H = bsn.FMRGrid3D(gas(m), m, m, m, DX, 5, 12, 5, 12, 5, 12, 2, G, **KW)
+    out["two levels"] = ([H.Uc, H.Uf], lambda n, t: bsn.fmr3d_run_steps(H, CFL, n_steps=n, t=t, precision=prec))
+    box = (5, 12, 5, 12, 5, 12, 2)
+    N = bsn.FMRHierarchy3D(gas(m), m, m, m, DX, (box, box), G, **KW)
+    out["levels"] = (list(N.levels), lambda n, t: bsn.fmr_nested_run_steps(N, CFL, n_steps=n, t=t, precision=prec))
+    B = bsn.FMRHierarchy3D(gas(m), m, m, m, DX, (box, box), G, **KW)
+    bh2 = [bsn.BlackHole((0.01, 0.0, 0.0), (0.0, 0.3, 0.0), 0.1, DX, 1e6, DX)]
+    out["nested"] = (list(B.levels), lambda n, t: bsn.coupled_nested_run_steps(B, bh2, -8 * DX, -8 * DX, -8 * DX, CFL,
+                                                                               n_steps=n, t=t, precision=prec))
+    return out, (U, H, N, B), (bhs, bh2)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_short_calls_equal_one_long_call(bsn, prec):
+    """One step a call (the first launched directly, the second captured, the
+    rest replayed), a call of one length between those of another, and all
+    steps in one call."""
+    bsn.set_tile(prec, 0)
+    loops, keep, holes = _loops(bsn, prec)
+    bh0 = [[bytes(b) for b in h] for h in holes]
+    start = {k: [a.clone() for a in s] for k, (s, _) in loops.items()}
+    got = {}
+    for name, (arrays, advance) in loops.items():
+        for calls in ((7,), (1,) * 7, (1, 1, 3, 2), (2, 2, 1, 1, 1)):
+            for a, b in zip(arrays, start[name]):
+                a.copy_(b)
+            for h, v in zip(holes, bh0):
+                for b, raw in zip(h, v):
+                    C.memmove(C.addressof(b), raw, len(raw))
+            t, done = 0.0, 0
+            for n in calls:
+                t, k = advance(n, t)
+                done += k
+            torch.cuda.synchronize()
+            res = [a.clone() for a in arrays]
+            if name in got:
+                assert (t, done) == got[name][0], (name, calls)
+                assert all(torch.equal(x, y) for x, y in zip(res, got[name][1])), (name, calls)
+            got[name] = ((t, done), res)
+    bsn.set_tile(prec, -1)
