@@ -166,9 +166,12 @@ bsn_status uniform_tiles_find(bsn_ctx* ctx, int prec, const f64::StageArgs& base
     return find_uniform(ctx, v, base, U, t.f[0]);
 }
 
-// stage-1 work of a probe, writing to scratch and recording nothing
+// stage-1 work of a probe, writing to scratch and recording nothing; a
+// right-hand side is timed as it runs, fluxes and all (it writes the same
+// values each time, and does not write its input)
 static f64::StageArgs probe_args(const f64::StageArgs& probe, double* scratch) {
     f64::StageArgs a = probe;
+    if (a.mode == 1) return a;
     a.Un = probe.Uin;
     a.Uout = scratch;
     a.mode = 0;

@@ -176,6 +176,7 @@ extern "C" bsn_status bsn_euler3d_rhs_f32(bsn_ctx* ctx, double* dU, double* Fx, 
     A.dU = dU;
     A.F[0] = Fx; A.F[1] = Fy; A.F[2] = Fz;
     A.mode = 1;
+    A.tune_class = TUNE_RHS;
     A.stiff_guard = ctx->stiff_guard;
     BSN_TRY(stage_launch(ctx, PREC_F32, A));
     // euler3d_rhs! floors U in place; the stage kernel floored its staged copies

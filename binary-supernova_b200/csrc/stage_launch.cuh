@@ -51,6 +51,9 @@ enum TuneClass {
     // (128^3 with a blast, FP64: a step that took a right-hand side's choice
     // was 2.95 ms instead of 1.76)
     TUNE_STEP = 7,
+    // right-hand sides, which store fluxes (FP32 128^3: 16x8x8 takes 444 us,
+    // the tile that wins a stage there 467)
+    TUNE_RHS = 8,
 };
 // The tile-choice code recorded for A's driver class and grid (-1: none yet).
 int tile_code(bsn_ctx* ctx, int precision, const f64::StageArgs& A);

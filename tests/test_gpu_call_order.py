@@ -239,3 +239,21 @@ def test_short_calls_equal_one_long_call(bsn, prec):
                 assert all(torch.equal(x, y) for x, y in zip(res, got[name][1])), (name, calls)
             got[name] = ((t, done), res)
     bsn.set_tile(prec, -1)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_right_hand_side_times_its_own_tiles(bsn, prec):
+    """A right-hand side stores fluxes and has another best tile than a stage:
+    the first one on a grid times the tiles, whatever stage came before."""
+    n = (40, 24, 24)
+    rhs = bsn.euler3d_rhs if prec == "f64" else bsn.euler3d_rhs_f32
+    U, V, F = bsn.state(*n), bsn.state(*n), bsn.flux_arrays(*n)
+    U[0], U[4] = 1.0, 1.0 / (G - 1)
+    bsn.set_tile(prec, -1)
+    bsn.euler3d_stage(V, U, U, *n, DX, DX, DX, 1e-3, G, 1, precision=prec, **KW)
+    counts = [bsn.launch_count()]
+    for _ in range(3):
+        rhs(V, *F, U, *n, DX, DX, DX, G, **KW)
+        counts.append(bsn.launch_count())
+    first, second, third = np.diff(counts)
+    assert second == third and first > second + bsn.tile_variants(prec)
