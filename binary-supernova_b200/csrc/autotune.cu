@@ -109,6 +109,40 @@ static bool uniform_tiles_apply(const f64::StageArgs& b) {
     return (long long)b.nx * b.ny * b.nz >= (1LL << 18);
 }
 
+static long long tiles_of(const TileVariant& v, const f64::StageArgs& b) {
+    return (long long)((b.nx + v.tx - 1) / v.tx) * ((b.ny + v.ty - 1) / v.ty) * ((b.nz + v.tz - 1) / v.tz);
+}
+
+// Whether to list, from the share of tiles listed lately.  The timing decides
+// at first; a state that then loses its uniform gas (a blast that fills the
+// box), or gets some, changes sides.  Eight steps on a state without uniform
+// gas after a first call on a blast, with the blast's choice kept and with this:
+// FP32 128^3 9.08 and 7.30 ms, learned 46.2 and 37.7, 256^3 FP32 61.6 and 55.0.
+// Listing pays for itself from some 15 % of uniform tiles on (with none, FP32
+// lists cost 20 %, FP64 7 %, learned ones nothing: every tile forced, 128^3).
+static void follow(bsn_ctx* ctx, int prec, const f64::StageArgs& base) {
+    const auto key = tile_key(prec, base);
+    auto it = ctx->list_use.find(key);
+    if (it == ctx->list_use.end()) return;
+    bsn_ctx::ListUse& use = it->second;
+    if (use.word < 0 || use.list < 0 || use.plain < 0) return;
+    volatile unsigned int* word = ctx->listed_now + use.word;
+    const unsigned int n = *word;   // may arrive while the steps go on: taken at the next call then
+    if (n == ~0u) return;
+    *word = ~0u;
+    const float uniform = 1.f - (float)n / (float)tiles_of(variant(prec, use.list & (kTmaBit - 1)), base),
+                timed = 1.f - use.listed;
+    int& code = ctx->tile_choice[key];
+    const bool on = code & kListBit;
+    bool want = on;
+    if (on && uniform < 0.15f) want = use.list_won && uniform > 0.5f * timed;
+    if (!on && uniform > 0.3f) want = use.list_won || uniform > timed + 0.2f;
+    if (want != on) {
+        code = want ? use.list : use.plain;
+        ctx->tile_last[std::make_tuple(prec, base.nx, base.ny, base.nz)] = code;
+    }
+}
+
 bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int prec, f64::StageArgs& base, UniformTiles& t) {
     t.on = uniform_tiles_apply(base);
     if (t.on && base.tune_class == TUNE_GENERIC) base.tune_class = TUNE_STEP;
@@ -122,11 +156,8 @@ bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int prec, f64::StageArgs& base, U
     }
     if (t.on) {
         size_t tiles = 0;
-        for (int v = 0; v < variant_count(prec); ++v) {
-            const TileVariant q = variant(prec, v);
-            tiles = std::max(tiles, (size_t)((base.nx + q.tx - 1) / q.tx) * ((base.ny + q.ty - 1) / q.ty) *
-                                        ((base.nz + q.tz - 1) / q.tz));
-        }
+        for (int v = 0; v < variant_count(prec); ++v)
+            tiles = std::max(tiles, (size_t)tiles_of(variant(prec, v), base));
         tiles = (tiles + 255) / 256 * 256;
         // Room for every grid that the stage buffers have room for (per axis at
         // most 1/7 tile per stored cell of n + 6 for the longer tile edges, 1/4
@@ -145,6 +176,7 @@ bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int prec, f64::StageArgs& base, U
         for (int i = 0; i < 3; ++i) t.f[i] = f + 256 + (sizeof(int) + i) * tiles;
     }
     if (capturing) return BSN_OK;
+    t.able = t.on && ctx->forced_tile[prec] < 0;
     f64::StageArgs p = base;
     t.set(p, 0);
     double* scratch = nullptr;
@@ -153,7 +185,37 @@ bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int prec, f64::StageArgs& base, U
         BSN_TRY(st);
     }
     BSN_TRY(stage_autotune(ctx, prec, p, scratch));
+    if (t.able) follow(ctx, prec, base);
     t.on = t.on && (tile_code(ctx, prec, base) & kListBit);
+    return BSN_OK;
+}
+
+__global__ void count_listed_kernel(const unsigned char* uniform, int tiles, unsigned int* listed) {
+    unsigned int n = 0;
+    for (int i = threadIdx.x; i < tiles; i += blockDim.x) n += uniform[i] == 0;
+    atomicAdd(listed, n);
+}
+
+bsn_status uniform_tiles_note(bsn_ctx* ctx, int prec, const f64::StageArgs& base, const double* U,
+                              const UniformTiles& t) {
+    if (!t.able) return BSN_OK;
+    auto it = ctx->list_use.find(tile_key(prec, base));
+    if (it == ctx->list_use.end() || it->second.word < 0 || it->second.list < 0) return BSN_OK;
+    bsn_ctx::ListUse& use = it->second;
+    // listing steps know what they listed; the others look seldom: a pass over
+    // the state is 1-2 % of a step
+    const int every = (base.tune_class == TUNE_STEP ? 8 : 1) * (t.on ? 1 : 4);
+    if (++use.calls % every) return BSN_OK;
+    if (!t.on) {
+        const TileVariant v = variant(prec, use.list & (kTmaBit - 1));
+        BSN_CUDA(ctx, cudaMemsetAsync(t.count, 0, 6 * sizeof(unsigned int), ctx->stream));
+        BSN_TRY(find_uniform(ctx, v, base, U, t.f[0]));
+        prof_begin(ctx);
+        count_listed_kernel<<<1, 1024, 0, ctx->stream>>>(t.f[0], (int)tiles_of(v, base), t.count + 4);
+        BSN_TRY(launch_check(ctx, "count_listed_kernel"));
+    }
+    BSN_CUDA(ctx, cudaMemcpyAsync(ctx->listed_now + use.word, t.count + 4, sizeof(unsigned int),
+                                  cudaMemcpyDeviceToHost, ctx->stream));
     return BSN_OK;
 }
 
@@ -265,8 +327,9 @@ bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, d
     cudaEvent_t e0, e1;
     BSN_CUDA(ctx, cudaEventCreate(&e0));
     BSN_CUDA(ctx, cudaEventCreate(&e1));
-    int best = 0;
-    float best_ms = 1e30f;
+    int best = 0, plain = -1, list = -1;
+    float best_ms = 1e30f, plain_ms = 1e30f, list_ms = 1e30f;
+    unsigned int listed = 0;
     bool prof = ctx->profiling;
     ctx->profiling = false;
     bsn_status st = BSN_OK;
@@ -290,6 +353,14 @@ bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, d
             if (r > 0) ms = t < ms ? t : ms;
         }
         if (ms + extra < best_ms) { best_ms = ms + extra; best = code; }
+        if (!(code & kListBit)) {
+            if (ms < plain_ms) { plain_ms = ms; plain = code; }
+        } else if (ms < list_ms && st == BSN_OK) {
+            list_ms = ms;
+            list = code;
+            st = cuda_check(ctx, cudaMemcpy(&listed, a.list_count, sizeof(listed), cudaMemcpyDeviceToHost),
+                            "cudaMemcpy(autotune)");
+        }
         return st == BSN_OK;
     };
     for (int v = 0; v < nv && st == BSN_OK; ++v) {
@@ -310,6 +381,21 @@ bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, d
     cudaEventDestroy(e1);
     BSN_TRY(st);
     record(ctx, prec, probe, best);
+    if (list >= 0) {
+        constexpr int kWords = 64;
+        if (!ctx->listed_now && cudaMallocHost(&ctx->listed_now, kWords * sizeof(unsigned int)) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->listed_now = nullptr;   // the choice stays as timed
+        }
+        const int next = (int)ctx->list_use.size();
+        bsn_ctx::ListUse& use = ctx->list_use[key];
+        if (use.word < 0 && ctx->listed_now && next < kWords) use.word = next;
+        if (use.word >= 0) ctx->listed_now[use.word] = ~0u;
+        use.plain = plain;
+        use.list = list;
+        use.list_won = best & kListBit;
+        use.listed = (float)listed / (float)tiles_of(variant(prec, list & (kTmaBit - 1)), probe);
+    }
     return BSN_OK;
 }
 
@@ -386,6 +472,8 @@ extern "C" bsn_status bsn_ctx_set_tile(bsn_ctx* ctx, int precision, int variant)
         it = std::get<0>(it->first) == precision ? ctx->tile_last.erase(it) : std::next(it);
     for (auto it = ctx->settled.begin(); it != ctx->settled.end();)
         it = it->second == precision ? ctx->settled.erase(it) : std::next(it);
+    for (auto it = ctx->list_use.begin(); it != ctx->list_use.end(); ++it)   // the words stay with their grids
+        if (std::get<0>(it->first) == precision) it->second.list = it->second.plain = -1;
     return BSN_OK;
 }
 

@@ -43,6 +43,17 @@ struct bsn_ctx {
     int retime_class = -1;
     std::set<std::tuple<int, int, int, int, int>> retimed;
     std::set<std::pair<int, int>> settled;
+    // steps that may list uniform tiles (autotune.cu): the fastest choice
+    // without and with a list, which of them was faster when they were timed
+    // and at which share of listed tiles, and where later shares arrive: a
+    // word of pinned memory (none for grids past the array's end)
+    struct ListUse {
+        int plain = -1, list = -1, calls = 0, word = -1;
+        bool list_won = false;
+        float listed = 1.f;
+    };
+    std::map<std::tuple<int, int, int, int, int>, ListUse> list_use;
+    unsigned int* listed_now = nullptr;
     int forced_tile[3] = {-1, -1, -1};
     void* learned_state = nullptr;   // learned.cu: packed network parameters
     // graph-captured device time loop (run_steps.cu)

@@ -135,6 +135,7 @@ extern "C" bsn_status bsn_ctx_destroy(bsn_ctx* ctx) {
     for (void* p : ctx->slot_ptr)
         if (p) cudaFree(p);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    if (ctx->listed_now) cudaFreeHost(ctx->listed_now);
     fft_state_free(ctx);
     fft32_state_free(ctx);
     run_state_free(ctx);

@@ -239,7 +239,7 @@ bsn_status f64_rk3(bsn_ctx* ctx, StageArgs base, double* U, double dt, const dou
     double* B = (double*)slot(ctx, SLOT_B, bytes, &st); BSN_TRY(st);
     double* in[3] = {U, A, B};
     double* out[3] = {A, B, U};
-    UniformTiles uni;
+    UniformTiles uni;   // none kept with a potential per stage
     if (!phi_per_stage) {
         base.Uin = U;
         base.Un = U;
@@ -256,6 +256,7 @@ bsn_status f64_rk3(bsn_ctx* ctx, StageArgs base, double* U, double dt, const dou
         a.cfl_nan = cfl_nan;
         BSN_TRY(f64_launch_stage(ctx, a));
     }
+    BSN_TRY(uniform_tiles_note(ctx, PREC_F64, base, U, uni));
     return f64_ghost_combine(ctx, U, B, nullptr, base.nx, base.ny, base.nz, base.bc, dt, nullptr, nullptr);
 }
 

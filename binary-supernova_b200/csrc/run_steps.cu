@@ -107,6 +107,7 @@ bsn_status rk3_prec(bsn_ctx* ctx, f64::StageArgs base, double* U, double dt, int
         set_stage(a, s + 1, dt);
         BSN_TRY(stage_launch(ctx, prec, a));
     }
+    BSN_TRY(uniform_tiles_note(ctx, prec, base, U, uni));
     return f64_ghost_combine(ctx, U, B, nullptr, base.nx, base.ny, base.nz, base.bc, dt);
 }
 
@@ -298,8 +299,9 @@ extern "C" bsn_status bsn_run_steps(bsn_ctx* ctx, double* U, int nx, int ny, int
         return graph_replay(ctx, S->exec, S->kernels, n, t_end > 0.0, &r->done, S->flag_ev,
                          (volatile int*)(h + 8));
     };
-    BSN_TRY(advance(settle ? 1 : n_steps));
+    int left = n_steps;
     if (settle) {   // the tile re-timed on the state after the first step
+        BSN_TRY(advance(1));
         BSN_TRY(tile_retime(ctx, TUNE_RUN, precision, tune));
         if (tile_code(ctx, precision, base) != variant) {
             variant = tile_code(ctx, precision, base);
@@ -307,12 +309,32 @@ extern "C" bsn_status bsn_run_steps(bsn_ctx* ctx, double* U, int nx, int ny, int
             if (!direct) BSN_TRY(capture());
         }
         BSN_TRY(uniform_tiles_find(ctx, precision, base, U, uni));   // of the new tile, or over the re-timing's use
-        BSN_TRY(advance(n_steps - 1));
+        --left;
     }
-    BSN_CUDA(ctx, cudaMemcpyAsync(h, r, sizeof(Dev), cudaMemcpyDeviceToHost, ctx->stream));
-    BSN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     Dev d;
-    memcpy(&d, h, sizeof(Dev));
+    auto read = [&]() -> bsn_status {
+        BSN_CUDA(ctx, cudaMemcpyAsync(h, r, sizeof(Dev), cudaMemcpyDeviceToHost, ctx->stream));
+        BSN_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        memcpy(&d, h, sizeof(Dev));
+        return BSN_OK;
+    };
+    // long runs look between chunks of steps whether listing still pays
+    constexpr int kChunk = 128;
+    d.done = 0;
+    while (uni.able && left > kChunk && !d.done) {
+        BSN_TRY(advance(kChunk));
+        left -= kChunk;
+        BSN_TRY(uniform_tiles_note(ctx, precision, base, U, uni));
+        BSN_TRY(read());
+        BSN_TRY(tune());
+        if (tile_code(ctx, precision, base) == variant) continue;
+        variant = tile_code(ctx, precision, base);
+        BSN_TRY(capture());
+        BSN_TRY(uniform_tiles_find(ctx, precision, base, U, uni));
+    }
+    if (!d.done) BSN_TRY(advance(left));
+    if (n_steps > 0) BSN_TRY(uniform_tiles_note(ctx, precision, base, U, uni));
+    BSN_TRY(read());
     *t_inout = d.t;
     if (steps_done) *steps_done = d.steps;
     if (d.done == 2) return set_err(ctx, BSN_ERR_NONFINITE, "time step collapsed to 0 at t = %.17g (infinite signal speed)", d.t);

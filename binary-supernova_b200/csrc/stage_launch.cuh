@@ -79,6 +79,7 @@ struct UniformTiles {
     int* list = nullptr;              // the tiles a stage leaves to the stage kernel
     unsigned int* count = nullptr;    // list count and queue counter of each stage
     bool on = false;
+    bool able = false;                // this step may list, or not, as its state goes
     void set(f64::StageArgs& a, int s) const {   // stage s = 0, 1, 2
         if (!on) return;
         a.uni_in = f[s];
@@ -92,6 +93,10 @@ struct UniformTiles {
 // Room for them, and the tile choice of base's grid (autotuned where it may);
 // puts single steps into their class.
 bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int precision, f64::StageArgs& base, UniformTiles& t);
+// After a step or a loop's steps on U: how many tiles are listed now, for the
+// next uniform_tiles_prepare to go by (it waits for nothing).
+bsn_status uniform_tiles_note(bsn_ctx* ctx, int precision, const f64::StageArgs& base, const double* U,
+                              const UniformTiles& t);
 // Those of U, for the tile choice of base's grid, and cleared counts.
 bsn_status uniform_tiles_find(bsn_ctx* ctx, int precision, const f64::StageArgs& base, const double* U,
                               const UniformTiles& t);

@@ -257,3 +257,66 @@ def test_right_hand_side_times_its_own_tiles(bsn, prec):
         counts.append(bsn.launch_count())
     first, second, third = np.diff(counts)
     assert second == third and first > second + bsn.tile_variants(prec)
+
+
+def _rough(bsn, n):
+    """No uniform gas anywhere."""
+    U = bsn.state(*n)
+    w = 0.0
+    for ax, m in enumerate(U.shape[1:]):
+        x = torch.arange(m, device="cuda", dtype=torch.float64) * (2 * np.pi * (ax + 1) / (m - 2 * NG))
+        w = w + torch.sin(x).reshape([-1 if a == ax else 1 for a in range(3)])
+    U[0], U[4] = 1.0 + 0.2 * w, 2.0 + 0.4 * w
+    return U
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_listing_follows_the_state(bsn, prec):
+    """Steps and loops that listed uniform tiles stop when the state has none
+    left, and take it up again, with the same bits throughout."""
+    n, dt = (128, 128, 128), 1e-4
+    step = bsn.euler3d_step if prec == "f64" else bsn.euler3d_step_f32
+    calm, rough = _calm(bsn, n), _rough(bsn, n)
+    a = (slice(None),) + (slice(NG, -NG),) * 3
+    bsn.set_tile(prec, 0)
+    want = {}
+    for name, U0 in (("calm", calm), ("rough", rough)):
+        U = U0.clone()
+        step(U, *n, DX, DX, DX, dt, G, bc="periodic", **KW)
+        V = U0.clone()
+        bsn.run_steps(V, *n, DX, DX, DX, G, CFL, n_steps=2, bc="periodic", precision=prec, **KW)
+        want[name] = U, V
+    bsn.set_tile(prec, -1)
+    for name, U0, times, listed in (("calm", calm, 2, 3), ("rough", rough, 20, 0), ("calm", calm, 80, 3)):
+        for _ in range(times):
+            U = U0.clone()
+            step(U, *n, DX, DX, DX, dt, G, bc="periodic", **KW)
+            assert torch.equal(U[a], want[name][0][a])
+        U = U0.clone()
+        k, = _launches(bsn, ["uniform_stage_kernel"],
+                       lambda: step(U, *n, DX, DX, DX, dt, G, bc="periodic", **KW))
+        assert k == listed, name
+
+    def loop(U0, steps):
+        U = U0.clone()
+        c = bsn.launch_count()
+        bsn.run_steps(U, *n, DX, DX, DX, G, CFL, n_steps=steps, bc="periodic", precision=prec, **KW)
+        return U, bsn.launch_count() - c
+    bsn.set_tile(prec, -1)
+    per = {}
+    for name, U0, times in (("calm", calm, 4), ("rough", rough, 4), ("calm", calm, 12)):
+        for _ in range(times):
+            U, c = loop(U0, 2)
+            assert torch.equal(U[a], want[name][1][a])
+        per[name] = c
+    assert per["calm"] > per["rough"]          # a list takes a launch more per stage
+    # one long call that starts on the list and goes on without it
+    a_step = (loop(calm, 6)[1] - loop(calm, 2)[1]) / 4
+    long, c = loop(rough, 300)
+    assert c < 300 * a_step - 3 * 100
+    U = rough.clone()
+    t = 0.0
+    for _ in range(3):
+        t, _k = bsn.run_steps(U, *n, DX, DX, DX, G, CFL, n_steps=100, t=t, bc="periodic", precision=prec, **KW)
+    assert torch.equal(U[a], long[a])
+    bsn.set_tile(prec, -1)
