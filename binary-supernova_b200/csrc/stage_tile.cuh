@@ -1,15 +1,16 @@
 // stage_tile.cuh -- the fused RK3-stage kernel as a template over the stencil
-// physics (FP64 parity or FP32 fast) and the tile shape (chosen by the
-// autotuner).  Included only by the translation units that instantiate it:
-// hydro_f64.cu (FP64 physics, built with -fmad=false) and stage_fast.cu (FP32
-// physics, built with FMA contraction and approximate division/sqrt).
+// physics and the tile shape (chosen by the autotuner).  Included by the units
+// that instantiate it: stage_f64_lo.cu and stage_f64_hi.cu (FP64 physics, no
+// contraction), stage_fast.cu and stage_guarded.cu (FP32 stencils) and
+// learned.cu (learned weights), the last three with approximate division and
+// square root and every multiply-add written out.
 //
-// A CTA owns a TX x TY x TZ block of active cells.  For each sweep direction
-// it stages the block plus a 3-cell halo along that direction in shared memory
-// (SoA; floors applied in FP64 to active cells, ghost cells taken raw through
-// the boundary map or from a ghost buffer, the cell pressure computed once per
-// staged cell), computes every interface of the block once, and accumulates
-// the flux divergence of its cells in FP64 registers.  The epilogue adds the
+// A CTA owns a TX x TY x TZ block of active cells.  It stages the block and
+// the 3-cell halos of all three sweeps in shared memory once (SoA; floors
+// applied in FP64 to active cells, ghost cells taken raw through the boundary
+// map or from a ghost buffer, the cell pressure computed once per staged
+// cell), computes every interface of the block once, a sweep at a time, and
+// accumulates the flux divergence of its cells in FP64 registers.  The epilogue adds the
 // source terms in the driver's order (BH gravity, self-gravity, sinks), the
 // SSP-RK3 combine and the floors in FP64, stores the stage result and folds
 // the next CFL speed into a device-wide max.
@@ -269,7 +270,7 @@ template <class P, int TX, int TY, int TZ, int NT, int D, bool LED>
 __device__ void sweep(const f64::StageArgs& A, const Geom& G, const typename P::Consts& k, int a0, int b0, int c0,
                       typename P::real* sC, typename P::real* sF, unsigned char* psm,
                       double (&acc)[Shape<TX, TY, TZ>::NCELL / NT][5], bool quiet_cross, bool records, bool full,
-                      double* sled) {
+                      double* sled, unsigned int* nlist, unsigned short* list) {
     using S = Shape<TX, TY, TZ>;
     using real = typename P::real;
     constexpr int CPT = S::NCELL / NT;
@@ -323,11 +324,11 @@ __device__ void sweep(const f64::StageArgs& A, const Geom& G, const typename P::
     // FP64 from the state, so the main loop keeps its registers, and the
     // listed faces are spread over all threads of the block (they cluster: a
     // star's surface, a sink's surroundings)
-    __shared__ int s_nlist;
-    __shared__ int s_list[P::kDeferred ? NF : 1];
+    // (nlist, list: the block's, used by one sweep after another; the barrier
+    // at a sweep's start follows every use of the sweep before)
     auto plain_faces = [&]() {
         if constexpr (P::kDeferred) {
-            if (tid == 0) s_nlist = 0;
+            if (tid == 0) *nlist = 0;
             __syncthreads();
         }
         for (int f = tid; f < NF; f += NT) {
@@ -346,15 +347,15 @@ __device__ void sweep(const f64::StageArgs& A, const Geom& G, const typename P::
             real F[5];
             const bool defer = P::flux(c, k, D, F);
             if constexpr (P::kDeferred) {
-                if (defer) { s_list[atomicAdd(&s_nlist, 1)] = f; continue; }
+                if (defer) { list[atomicAdd(nlist, 1u)] = (unsigned short)f; continue; }
             }
             emit(f, fx, fy, fz, F);
         }
         if constexpr (P::kDeferred) {
             __syncthreads();
-            const int nst = s_nlist;   // read by every thread before the next sweep resets it
+            const int nst = (int)*nlist;   // read by every thread before the next sweep resets it
             for (int i = tid; i < nst; i += NT) {
-                const int f = s_list[i];
+                const int f = list[i];
                 const int fx = f % FX, r = f / FX, fy = r % FY, fz = r / FY;
                 double F64[5];
                 face_flux_f64<D>(A, o[0] + fx, o[1] + fy, o[2] + fz, F64);
@@ -449,7 +450,9 @@ struct TmaSmem {
                                              127) / 128 * 128);
     static constexpr int in_faces(int rawb) { return FACE_BYTES >= 2 * rawb ? 2 : (FACE_BYTES >= rawb ? 1 : 0); }
     static constexpr int bytes_for(int rawb) { return APPEND_OFF + (2 - in_faces(rawb)) * rawb; }
-    static constexpr int BUDGET = 233472 / MINB - 2048;   // per-CTA smem that keeps MINB CTAs on an SM
+    // per-CTA dynamic smem that keeps MINB CTAs on an SM, beside the system's
+    // 1 KB, the deferred faces' list and up to 1 KB of other static smem
+    static constexpr int BUDGET = 233472 / MINB - 2048 - (P::kDeferred && P::kCols == 5 ? 2 * S::NFACE : 0);
     static constexpr int CAP = bytes_for(tma::Chunks<TX, TY, TZ, tma::kChunkCap>::RAWB) <= BUDGET
                                    ? tma::kChunkCap
                                    : FACE_BYTES / 2 / 128 * 128;
@@ -811,6 +814,17 @@ __device__ __forceinline__ bool stage_block(const f64::StageArgs& A, int a0, int
         }
     }
     const bool full = a0 + TX <= A.nx && b0 + TY <= A.ny && c0 + TZ <= A.nz;
+    static_assert(S::NFACE <= 65536, "face indices of 16 bits");
+    // Faces deferred to a sweep's second pass.  Where their list would cost a
+    // CTA per SM (FP64 16x8x4 at two: 880 bytes are left) it lies in the staged
+    // column of E, whose halo cells nothing reads.
+    constexpr int kDyn = (P::kCols * S::NCROSS + 5 * S::NFACE) * (int)sizeof(real) + 16, kRest = 1024 + 512;
+    constexpr bool kListInHalo = P::kDeferred && P::kCols == 6 && (kDyn + kRest) * MINB <= 233472 &&
+                                 (kDyn + kRest + 2 * S::NFACE) * MINB > 233472;
+    static_assert(!kListInHalo || sizeof(real) * (S::NCROSS - S::NCELL) >= 2 * S::NFACE, "the halos hold the list");
+    __shared__ unsigned int nlist;
+    __shared__ unsigned short slist[P::kDeferred && !kListInHalo ? S::NFACE : 1];
+    unsigned short* list = kListInHalo ? reinterpret_cast<unsigned short*>(sC + 4 * S::NCROSS + S::NCELL) : slist;
     if (uniform) {
         // -(F - F) / dx - (F - F) / dy - (F - F) / dz of finite fluxes
         const double none = (-(0.0) * A.idx - 0.0 * A.idy) - 0.0 * A.idz;
@@ -819,9 +833,9 @@ __device__ __forceinline__ bool stage_block(const f64::StageArgs& A, int a0, int
 #pragma unroll
             for (int q = 0; q < 5; ++q) acc[m][q] = none;
     } else {
-        sweep<P, TX, TY, TZ, NT, 0, LED>(A, G, k, a0, b0, c0, sC, sF, psm, acc, quiet[0], face_out, full, sled);
-        sweep<P, TX, TY, TZ, NT, 1, LED>(A, G, k, a0, b0, c0, sC, sF, psm, acc, quiet[1], face_out, full, sled);
-        sweep<P, TX, TY, TZ, NT, 2, LED>(A, G, k, a0, b0, c0, sC, sF, psm, acc, quiet[2], face_out, full, sled);
+        sweep<P, TX, TY, TZ, NT, 0, LED>(A, G, k, a0, b0, c0, sC, sF, psm, acc, quiet[0], face_out, full, sled, &nlist, list);
+        sweep<P, TX, TY, TZ, NT, 1, LED>(A, G, k, a0, b0, c0, sC, sF, psm, acc, quiet[1], face_out, full, sled, &nlist, list);
+        sweep<P, TX, TY, TZ, NT, 2, LED>(A, G, k, a0, b0, c0, sC, sF, psm, acc, quiet[2], face_out, full, sled, &nlist, list);
     }
 
     const double dt = A.dt_dev ? *A.dt_dev : A.dt;
