@@ -2,17 +2,19 @@
 //
 // The FP64 path's bits are IEEE division's, and a face of the reference
 // scheme has some 85 of them: 12 per reconstructed field, several by the same
-// density.  A compiled `a / b` is an opaque sequence with its own range checks
-// and a call for the rare cases, which costs about 25 instructions and keeps
-// the compiler from interleaving neighbouring divisions; it made up most of
-// the FP64 stage kernel's instructions.  Here the reciprocal of a denominator
-// is formed once and every quotient by it takes three more operations:
+// density.  Here the reciprocal of a denominator is formed once and every
+// quotient by it takes three more operations:
 //   * recip_rn: the hardware's reciprocal approximation (PTX
-//     rcp.approx.ftz.f64), one third-order and one second-order
-//     Newton-Raphson step.  The first is rounded upward: the second then
-//     rounds correctly for every mantissa, also the one of all ones (as in
-//     0.1 + 0.6 + 0.3, the WENO weights' sum in smooth flow), whose reciprocal
-//     lies just above a tie;
+//     rcp.approx.ftz.f64) refined by the geometric series of its residual e =
+//     1 - b y, 1 / b = y (1 + e + e^2 + ...): first to e^2, then to e, each
+//     in fused operations (Cornea-Hasegan, Golliver and Markstein, "Correctness
+//     proofs outline for Newton-Raphson based floating-point divide and square
+//     root algorithms", 14th IEEE Symposium on Computer Arithmetic, 1999; the
+//     last step rounds correctly from a y within an ulp by Markstein, below,
+//     unless b's significand is all ones, as in 0.1 + 0.6 + 0.3, the WENO
+//     weights' sum in smooth flow).  The first step here is rounded upward:
+//     the reciprocal of an all-ones significand lies just above a tie, and from
+//     above the last step reaches its upper neighbour;
 //   * quot: q = a y, then the remainder a - b q (exact in one fused
 //     operation) times y added back.  This rounds correctly when y is the
 //     rounded reciprocal and no intermediate leaves the normal range
