@@ -497,10 +497,26 @@ struct F32Learned {
         uint4* dst = (uint4*)psm;                 // policy_smem: 16-byte aligned
         for (int i = threadIdx.x; i < 2 * learned::PK_BYTES / 16; i += nt) dst[i] = src[i];
     }
-    // the FP32 path's end of a face
-    __device__ __forceinline__ static void finish(const float (&c)[6][6], const Consts& k, const float (&L)[5],
-                                                  const float (&Rv)[5], float (&F)[5], int D) {
-        f32::finish_face(c, L, Rv, k.g, k.gm1, k.inv_gm1, k.gg, D, F);
+    // The FP32 path's end of a face, side by side instead of packed: the same
+    // bits, and fewer registers live around the network's tiles.  Learned steps
+    // without uniform gas, packed and so: 128x96x80 2.39 and 2.35 ms, 256^3 32.9
+    // and 32.6, 48^3 0.439 and 0.443.
+    __device__ static void finish(const float (&c)[6][6], const Consts& k, const float (&L)[5], const float (&Rv)[5],
+                                  float (&F)[5], int D) {
+        const float Pm = fmaxf(fmaxf(fmaxf(c[1][5], c[2][5]), c[3][5]), c[4][5]);
+        const float PL = fminf(fmaxf(L[4], 0.0f), fmaxf(c[0][5], Pm)), PR = fminf(fmaxf(Rv[4], 0.0f), fmaxf(Pm, c[5][5]));
+        const float EL = f32::EL_from_P(PL, L[0], L[1], L[2], L[3], k.inv_gm1);
+        const float ER = f32::EL_from_P(PR, Rv[0], Rv[1], Rv[2], Rv[3], k.inv_gm1);
+        // (normal, t1, t2) = (x, y, z), (y, x, z), (z, x, y)
+        float Fr[5];
+        f32::hllc_normal(L[0], D == 0 ? L[1] : (D == 1 ? L[2] : L[3]), D == 0 ? L[2] : L[1], D == 2 ? L[2] : L[3], EL,
+                         Rv[0], D == 0 ? Rv[1] : (D == 1 ? Rv[2] : Rv[3]), D == 0 ? Rv[2] : Rv[1],
+                         D == 2 ? Rv[2] : Rv[3], ER, k.g, k.gm1, k.gg, Fr);
+        F[0] = Fr[0];
+        F[1] = D == 0 ? Fr[1] : Fr[2];
+        F[2] = D == 0 ? Fr[2] : (D == 1 ? Fr[1] : Fr[3]);
+        F[3] = D == 2 ? Fr[1] : Fr[3];
+        F[4] = Fr[4];
     }
     // One interface per lane; every lane of the warp calls this (valid or not).
     // c[cell][col]: cols 0-3 rho, m_x, m_y, m_z, col 4 E, col 5 P; the
