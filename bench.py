@@ -47,6 +47,8 @@ sys.path.insert(0, os.path.join(ROOT, "oracle"))
 NG = 3
 GAMMA = 5.0 / 3.0
 CFL = 0.4
+# DRAM bytes of an RK3 stage at Sedov 128^3, t = 0.025 (ncu: a step's launches, the flag pass included, / 3)
+TRAFFIC_128 = {"f64": 139.8e6, "f32": 128.4e6, "learned": 133.0e6}
 T_MID = 0.025     # start of the timed steps (Sedov run to t = 0.05)
 T_END = 0.05
 METRIC = "cell-updates/s per RK3 step (Sedov 3D, WENO5-Z+HLLC+SSP-RK3)"   # both arms
@@ -849,30 +851,30 @@ def run_bsn(args, rank, world):
         log(f"{p_}: {ms_other[p_] / args.steps:.3f} ms/step")
     value = world * ncell * args.steps / (ms / 1e3)
 
-    # roofline of the dominant kernel: stage-kernel launches timed with CUDA
-    # events around each launch (per-step entry point, same kernels)
+    # roofline of the dominant kernels: a stage's launches timed with CUDA
+    # events around each (per-step entry point, same kernels).  A stage may be
+    # several launches: uniform tiles apart, the listed ones, a learned stage's
+    # screen; single steps also find the uniform tiles, once per three stages
     kname = {"f32": "stage_kernel_f32", "f64": "stage_kernel", "learned": "stage_kernel_learned"}[prec]
     step_fn = {"f32": bsn.euler3d_step_f32, "f64": bsn.euler3d_step, "learned": bsn.euler3d_step_learned}[prec]
     Up = Ud.clone()
     dt0 = bsn.cfl_dt_3d(Up, n, n, n, dx, dx, dx, GAMMA, CFL)
     step_fn(Up, n, n, n, dx, dx, dx, dt0, GAMMA, **kw)
     bsn.set_profiling(True)
-    for _ in range(3):
+    prof_steps = 3
+    for _ in range(prof_steps):
         step_fn(Up, n, n, n, dx, dx, dx, dt0, GAMMA, **kw)
-    tot, cnt = bsn.kernel_time(kname)
-    if prec != "learned":   # the stage kernel with TMA staging, where the grid allows it
-        t_, c_ = bsn.kernel_time(kname + "_tma")
-        if c_:
-            tot, cnt, kname = tot + t_, cnt + c_, kname + "_tma"
-    if prec == "learned":   # a learned stage is a screening launch plus the learned launch
-        tot += bsn.kernel_time("stage_kernel_learned_screen")[0]
-        kname = "stage_kernel_learned_screen + stage_kernel_learned"
+    parts = {k_: bsn.kernel_time(k_) for k_ in ("uniform_tiles_kernel", "uniform_stage_kernel", kname + "_screen",
+                                                kname, kname + "_tma")}
     bsn.set_profiling(False)
+    tot = sum(t_ for t_, _ in parts.values())
+    kname = " + ".join(k_ for k_, (_, c_) in parts.items() if c_)
+    cnt = 3 * prof_steps
     t_stage = tot / max(cnt, 1) / 1e3
     alg_bytes = 40 * 8 * ncell / 3.0     # 40 FP64 state words per cell per RK3 step, 3 stage launches
-    # DRAM bytes of one stage-1 launch (learned: its screening and learned launches) from an ncu
-    # capture at 128^3 (t = 0.025), scaled by the cell count (profiles/stage_kernel_*_sedov128_ncu.md)
-    traffic_128 = {"learned": 134.1e6, "f32": 133.7e6, "f64": 133.1e6}.get(prec)
+    # DRAM bytes of one step's launches over its three stages, from an ncu capture at 128^3
+    # (t = 0.025), scaled by the cell count (profiles/stage_kernels_sedov128_ncu.md)
+    traffic_128 = TRAFFIC_128.get(prec)
     traffic = traffic_128 * ncell / 128 ** 3 if traffic_128 else None
     hbm, hbm_kind = peaks()
     achieved = alg_bytes / t_stage / 1e9
@@ -957,8 +959,9 @@ def run_bsn(args, rank, world):
             "poisson": poisson,
             "roofline": {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": hbm, "peak_kind": hbm_kind,
                          "unit": "GB/s", "frac": achieved / hbm, "traffic": traffic,
-                         "traffic_note": "DRAM read+write of one stage-1 launch, ncu at 128^3 scaled by cells",
+                         "traffic_note": "DRAM read+write of a step's stage launches / 3, ncu at 128^3 scaled by cells",
                          "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": t_stage * 1e3,
+                         "launch": "one RK3 stage, all its kernels",
                          "note": "the fused stencil kernel is FP-pipe bound (FP32/FP64), not HBM bound; "
                                  "HBM fraction of the algorithmic 40 words/cell-step"},
             "fp_pipe": fp_pipe(prec, ms, ms_other, ncell * world * args.steps, peak_fp),
