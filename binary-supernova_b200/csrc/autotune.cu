@@ -109,6 +109,13 @@ static bool uniform_tiles_apply(const f64::StageArgs& b) {
     return (long long)b.nx * b.ny * b.nz >= (1LL << 18);
 }
 
+// one block: the tiles that are not uniform, added to *listed
+__global__ void count_listed_kernel(const unsigned char* uniform, int tiles, unsigned int* listed) {
+    unsigned int n = 0;
+    for (int i = threadIdx.x; i < tiles; i += blockDim.x) n += uniform[i] == 0;
+    atomicAdd(listed, n);
+}
+
 static long long tiles_of(const TileVariant& v, const f64::StageArgs& b) {
     return (long long)((b.nx + v.tx - 1) / v.tx) * ((b.ny + v.ty - 1) / v.ty) * ((b.nz + v.tz - 1) / v.tz);
 }
@@ -118,8 +125,9 @@ static long long tiles_of(const TileVariant& v, const f64::StageArgs& b) {
 // box), or gets some, changes sides.  Eight steps on a state without uniform
 // gas after a first call on a blast, with the blast's choice kept and with this:
 // FP32 128^3 9.08 and 7.30 ms, learned 46.2 and 37.7, 256^3 FP32 61.6 and 55.0.
-// Listing pays for itself from some 15 % of uniform tiles on (with none, FP32
-// lists cost 20 %, FP64 7 %, learned ones nothing: every tile forced, 128^3).
+// Listing pays for itself once it leaves out some 15 % of the tiles (with none,
+// FP32 lists cost 20 %, FP64 7 %, learned ones nothing: every tile forced,
+// 128^3).  A side that turned out wrong has to be exceeded by a fifth.
 static void follow(bsn_ctx* ctx, int prec, const f64::StageArgs& base) {
     const auto key = tile_key(prec, base);
     auto it = ctx->list_use.find(key);
@@ -130,13 +138,21 @@ static void follow(bsn_ctx* ctx, int prec, const f64::StageArgs& base) {
     const unsigned int n = *word;   // may arrive while the steps go on: taken at the next call then
     if (n == ~0u) return;
     *word = ~0u;
-    const float uniform = 1.f - (float)n / (float)tiles_of(variant(prec, use.list & (kTmaBit - 1)), base),
-                timed = 1.f - use.listed;
+    // of a list the share of tiles it left out, else of uniform tiles (more:
+    // those beside others are listed too)
+    const float share = 1.f - (float)n / (float)tiles_of(variant(prec, use.list & (kTmaBit - 1)), base);
     int& code = ctx->tile_choice[key];
     const bool on = code & kListBit;
     bool want = on;
-    if (on && uniform < 0.15f) want = use.list_won && uniform > 0.5f * timed;
-    if (!on && uniform > 0.3f) want = use.list_won || uniform > timed + 0.2f;
+    if (on && use.left_out < 0.f) use.left_out = share;   // of the state it was timed on
+    if (on && share < 0.15f && (!use.list_won || share < 0.5f * use.left_out)) {
+        want = false;
+        use.no_gain = std::min(std::max(share, use.taken_at), 0.6f);
+    }
+    if (!on && share > std::max(use.no_gain + 0.2f, 0.3f)) {
+        want = true;
+        use.taken_at = share;
+    }
     if (want != on) {
         code = want ? use.list : use.plain;
         ctx->tile_last[std::make_tuple(prec, base.nx, base.ny, base.nz)] = code;
@@ -190,12 +206,6 @@ bsn_status uniform_tiles_prepare(bsn_ctx* ctx, int prec, f64::StageArgs& base, U
     return BSN_OK;
 }
 
-__global__ void count_listed_kernel(const unsigned char* uniform, int tiles, unsigned int* listed) {
-    unsigned int n = 0;
-    for (int i = threadIdx.x; i < tiles; i += blockDim.x) n += uniform[i] == 0;
-    atomicAdd(listed, n);
-}
-
 bsn_status uniform_tiles_note(bsn_ctx* ctx, int prec, const f64::StageArgs& base, const double* U,
                               const UniformTiles& t) {
     if (!t.able) return BSN_OK;
@@ -205,7 +215,7 @@ bsn_status uniform_tiles_note(bsn_ctx* ctx, int prec, const f64::StageArgs& base
     // listing steps know what they listed; the others look seldom: a pass over
     // the state is 1-2 % of a step
     const int every = (base.tune_class == TUNE_STEP ? 8 : 1) * (t.on ? 1 : 4);
-    if (++use.calls % every) return BSN_OK;
+    if (use.calls++ % every) return BSN_OK;
     if (!t.on) {
         const TileVariant v = variant(prec, use.list & (kTmaBit - 1));
         BSN_CUDA(ctx, cudaMemsetAsync(t.count, 0, 6 * sizeof(unsigned int), ctx->stream));
@@ -329,7 +339,7 @@ bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, d
     BSN_CUDA(ctx, cudaEventCreate(&e1));
     int best = 0, plain = -1, list = -1;
     float best_ms = 1e30f, plain_ms = 1e30f, list_ms = 1e30f;
-    unsigned int listed = 0;
+    unsigned int mixed = 0;   // of its tiles, those that are not uniform
     bool prof = ctx->profiling;
     ctx->profiling = false;
     bsn_status st = BSN_OK;
@@ -358,8 +368,11 @@ bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, d
         } else if (ms < list_ms && st == BSN_OK) {
             list_ms = ms;
             list = code;
-            st = cuda_check(ctx, cudaMemcpy(&listed, a.list_count, sizeof(listed), cudaMemcpyDeviceToHost),
-                            "cudaMemcpy(autotune)");
+            cudaMemsetAsync(a.list_count, 0, sizeof(unsigned int), ctx->stream);
+            count_listed_kernel<<<1, 1024, 0, ctx->stream>>>(
+                a.uni_in, (int)tiles_of(variant(prec, code & (kTmaBit - 1)), a), a.list_count);
+            cudaMemcpyAsync(&mixed, a.list_count, sizeof(mixed), cudaMemcpyDeviceToHost, ctx->stream);
+            st = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize(autotune)");
         }
         return st == BSN_OK;
     };
@@ -394,7 +407,11 @@ bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, d
         use.plain = plain;
         use.list = list;
         use.list_won = best & kListBit;
-        use.listed = (float)listed / (float)tiles_of(variant(prec, list & (kTmaBit - 1)), probe);
+        const float tiles = (float)tiles_of(variant(prec, list & (kTmaBit - 1)), probe);
+        use.left_out = -1.f;
+        use.no_gain = use.list_won ? 0.f : 1.f - (float)mixed / tiles;
+        use.taken_at = 0.f;
+        use.calls = 0;
     }
     return BSN_OK;
 }

@@ -44,13 +44,15 @@ struct bsn_ctx {
     std::set<std::tuple<int, int, int, int, int>> retimed;
     std::set<std::pair<int, int>> settled;
     // steps that may list uniform tiles (autotune.cu): the fastest choice
-    // without and with a list, which of them was faster when they were timed
-    // and at which share of listed tiles, and where later shares arrive: a
-    // word of pinned memory (none for grids past the array's end)
+    // without and with a list, whether the list was faster when they were timed
+    // and the share of tiles it then left out (below 0: not known yet), the
+    // share of uniform tiles up to which it is known not to pay, the one it was
+    // last taken up at, and where later counts arrive: a word of pinned memory
+    // (none for grids past the array's end)
     struct ListUse {
         int plain = -1, list = -1, calls = 0, word = -1;
         bool list_won = false;
-        float listed = 1.f;
+        float left_out = -1.f, no_gain = 0.f, taken_at = 0.f;
     };
     std::map<std::tuple<int, int, int, int, int>, ListUse> list_use;
     unsigned int* listed_now = nullptr;

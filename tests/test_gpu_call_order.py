@@ -320,3 +320,29 @@ def test_listing_follows_the_state(bsn, prec):
         t, _k = bsn.run_steps(U, *n, DX, DX, DX, G, CFL, n_steps=100, t=t, bc="periodic", precision=prec, **KW)
     assert torch.equal(U[a], long[a])
     bsn.set_tile(prec, -1)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("share", [0.3, 0.6, 0.85])
+def test_listing_is_steady_on_one_state(bsn, prec, share):
+    """Whether a list pays was timed on this state: steps that start from it
+    again and again do not change sides, whatever share of it is uniform."""
+    n = (150, 101, 67)
+    step = bsn.euler3d_step if prec == "f64" else bsn.euler3d_step_f32
+    U0 = _rough(bsn, n)
+    k = NG + int(n[1] * (1 - share))
+    U0[:, :, k:-NG] = 0.0
+    U0[0, :, k:-NG], U0[4, :, k:-NG] = 1.0, 2.0
+    U, seen = U0.clone(), set()
+    bsn.set_tile(prec, -1)
+
+    def one():
+        U.copy_(U0)
+        step(U, *n, DX, DX, DX, 1e-4, G, bc="periodic", **KW)
+    for _ in range(8):
+        one()
+        seen.add((_launches(bsn, ["uniform_stage_kernel"], one)[0], bsn.get_tile(*n, prec)))
+        for _ in range(12):
+            one()
+    assert len(seen) == 1, seen
+    bsn.set_tile(prec, -1)
