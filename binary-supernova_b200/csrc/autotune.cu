@@ -263,8 +263,9 @@ static f64::StageArgs probe_args(const f64::StageArgs& probe, double* scratch) {
 // The drivers whose stages run over several grids at once: one choice for all
 // of them, timed as they run, in one launch over every level.  (Timed level by
 // level, levels of one size share the first one's choice: three 128^3 levels
-// of the binary star took the coarse level's 8x8x8, 16.9 ms per step, where
-// 16x16x8 of 512 threads takes 14.9.)
+// of the binary star took the coarse level's 8x8x8, 16.9 ms a step; timed
+// without their flux registers, two FP64 levels of 64^3 took 16x8x4 in three
+// calls of four, 12.08 ms for eight steps where 16x8x8 takes 11.77.)
 bsn_status stage_autotune_batch(bsn_ctx* ctx, int prec, const f64::StageArgs* probes, double* const* scratch, int n) {
     if (n < 1 || n > f64::MAXLEV) return set_err(ctx, BSN_ERR_ARG, "batch of %d levels", n);
     bool known = true;
@@ -287,6 +288,10 @@ bsn_status stage_autotune_batch(bsn_ctx* ctx, int prec, const f64::StageArgs* pr
         }
         if (probes[l].tune_class == ctx->retime_class) ctx->retimed.insert(tile_key(prec, probes[l]));
         B.lv[l] = probe_args(probes[l], scratch[l]);
+        // the fluxes that levels record, too: the loops clear the registers
+        // before they use them and write the boundary faces anew
+        B.lv[l].use_reg = probes[l].use_reg;
+        B.lv[l].use_bnd = probes[l].use_bnd;
     }
     int best = 0;
     if (ctx->forced_tile[prec] >= 0) {
