@@ -457,7 +457,8 @@ struct State {
 // from the network (BF16 tensor cores) where the stencil is smooth.
 namespace tile {
 
-struct F32Learned {
+template <bool PACKED>
+struct F32LearnedT {
     static constexpr bool kDeferred = false;   // the warp path reconstructs all faces in FP32
     using real = float;
     static constexpr bool kCenterFromSmem = false;
@@ -497,12 +498,19 @@ struct F32Learned {
         uint4* dst = (uint4*)psm;                 // policy_smem: 16-byte aligned
         for (int i = threadIdx.x; i < 2 * learned::PK_BYTES / 16; i += nt) dst[i] = src[i];
     }
-    // The FP32 path's end of a face, side by side instead of packed: the same
-    // bits, and fewer registers live around the network's tiles.  Learned steps
-    // without uniform gas, packed and so: 128x96x80 2.39 and 2.35 ms, 256^3 32.9
-    // and 32.6, 48^3 0.439 and 0.443.
-    __device__ static void finish(const float (&c)[6][6], const Consts& k, const float (&L)[5], const float (&Rv)[5],
-                                  float (&F)[5], int D) {
+    // The FP32 path's end of a face: packed, or side by side with the same bits
+    // and fewer registers live around the network's tiles.  Where every block
+    // of the launch is one that the screen listed, side by side is faster:
+    // learned steps without uniform gas, packed and so, 128x96x80 2.39 and 2.35
+    // ms, 256^3 32.9 and 32.6, 48^3 0.439 and 0.443; over all blocks of a level
+    // packed is: two levels of 64^3, eight steps, 10.67 and 10.80 ms.
+    __device__ __forceinline__ static void finish(const float (&c)[6][6], const Consts& k, const float (&L)[5],
+                                                  const float (&Rv)[5], float (&F)[5], int D) {
+        if constexpr (PACKED) f32::finish_face(c, L, Rv, k.g, k.gm1, k.inv_gm1, k.gg, D, F);
+        else finish_sides(c, k, L, Rv, F, D);
+    }
+    __device__ static void finish_sides(const float (&c)[6][6], const Consts& k, const float (&L)[5],
+                                        const float (&Rv)[5], float (&F)[5], int D) {
         const float Pm = fmaxf(fmaxf(fmaxf(c[1][5], c[2][5]), c[3][5]), c[4][5]);
         const float PL = fminf(fmaxf(L[4], 0.0f), fmaxf(c[0][5], Pm)), PR = fminf(fmaxf(Rv[4], 0.0f), fmaxf(Pm, c[5][5]));
         const float EL = f32::EL_from_P(PL, L[0], L[1], L[2], L[3], k.inv_gm1);
@@ -671,6 +679,8 @@ struct F32Learned {
         return false;
     }
 };
+using F32Learned = F32LearnedT<true>;
+using F32LearnedListed = F32LearnedT<false>;
 
 // The screening launch of the learned stage: the FP32 path's plain stencils
 // for every block whose three sweeps are uniform by F32Learned's test (no
@@ -724,7 +734,7 @@ bsn_status launch_learned(bsn_ctx* ctx, const f64::StageArgs& A0) {
     }
     A.list = A.split_list;
     A.list_count = A.split_count;
-    return tile::launch_list<tile::F32Learned, TX, TY, TZ, NT, MINB, false>(ctx, A, smem_l, "stage_kernel_learned");
+    return tile::launch_list<tile::F32LearnedListed, TX, TY, TZ, NT, MINB, false>(ctx, A, smem_l, "stage_kernel_learned");
 }
 }  // namespace
 
