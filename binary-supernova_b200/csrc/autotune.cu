@@ -124,7 +124,7 @@ static long long tiles_of(const TileVariant& v, const f64::StageArgs& b) {
 // at first; a state that then loses its uniform gas (a blast that fills the
 // box), or gets some, changes sides.  Eight steps on a state without uniform
 // gas after a first call on a blast, with the blast's choice kept and with this:
-// FP32 128^3 9.08 and 7.30 ms, learned 46.2 and 37.7, 256^3 FP32 61.6 and 55.0.
+// FP32 128^3 9.00 and 7.29 ms, learned 47.5 and 37.7, 256^3 FP32 61.6 and 54.7.
 // Listing pays for itself once it leaves out some 15 % of the tiles (with none,
 // FP32 lists cost 20 %, FP64 7 %, learned ones nothing: every tile forced,
 // 128^3).  A side that turned out wrong has to be exceeded by a fifth.
