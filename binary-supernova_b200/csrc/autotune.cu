@@ -6,7 +6,8 @@
 // every tile variant on stage-1 work (reading the caller's state, writing a
 // scratch array), with each staging the grid allows, times two launches of
 // each with CUDA events after one warm-up, and keeps the fastest for the life
-// of the context.  Every variant and staging gives bit-identical results (FP64
+// of the context (of steps that may list uniform tiles, the fastest with and
+// without a list: follow).  Every variant and staging gives bit-identical results (FP64
 // by the reference's arithmetic, FP32 by its written-out multiply-adds), so
 // the choice never changes a result.  The choice is stored as a code: the
 // variant index plus kTmaBit when the TMA form won.
@@ -125,9 +126,12 @@ static long long tiles_of(const TileVariant& v, const f64::StageArgs& b) {
 // box), or gets some, changes sides.  Eight steps on a state without uniform
 // gas after a first call on a blast, with the blast's choice kept and with this:
 // FP32 128^3 9.00 and 7.29 ms, learned 47.5 and 37.7, 256^3 FP32 61.6 and 54.7.
-// Listing pays for itself once it leaves out some 15 % of the tiles (with none,
-// FP32 lists cost 20 %, FP64 7 %, learned ones nothing: every tile forced,
-// 128^3).  A side that turned out wrong has to be exceeded by a fifth.
+// Listing pays for itself once it leaves out a quarter of the tiles: with 0, 20,
+// 40 and 60 % of a 128^3 box in a uniform slab, us a stage, the best list and
+// the best tile without, FP32 351, 331, 288, 235 and 294 throughout, FP64 959,
+// 1140, 1029, 835 and 905, 1044, 1082, 1086 (the slab's neighbours are listed
+// too: two tiles of its eight at 40 %).  A side that turned out wrong has to be
+// exceeded by a fifth.
 static void follow(bsn_ctx* ctx, int prec, const f64::StageArgs& base) {
     const auto key = tile_key(prec, base);
     auto it = ctx->list_use.find(key);
@@ -145,11 +149,11 @@ static void follow(bsn_ctx* ctx, int prec, const f64::StageArgs& base) {
     const bool on = code & kListBit;
     bool want = on;
     if (on && use.left_out < 0.f) use.left_out = share;   // of the state it was timed on
-    if (on && share < 0.15f && (!use.list_won || share < 0.5f * use.left_out)) {
+    if (on && share < 0.25f && (!use.list_won || share < 0.5f * use.left_out)) {
         want = false;
         use.no_gain = std::min(std::max(share, use.taken_at), 0.6f);
     }
-    if (!on && share > std::max(use.no_gain + 0.2f, 0.3f)) {
+    if (!on && share > std::max(use.no_gain + 0.2f, 0.45f)) {
         want = true;
         use.taken_at = share;
     }
@@ -344,7 +348,7 @@ bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, d
     BSN_CUDA(ctx, cudaEventCreate(&e1));
     int best = 0, plain = -1, list = -1;
     float best_ms = 1e30f, plain_ms = 1e30f, list_ms = 1e30f;
-    unsigned int mixed = 0;   // of its tiles, those that are not uniform
+    unsigned int listed = 0, mixed = 0;   // of its tiles, those listed, and those that are not uniform
     bool prof = ctx->profiling;
     ctx->profiling = false;
     bsn_status st = BSN_OK;
@@ -373,6 +377,7 @@ bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, d
         } else if (ms < list_ms && st == BSN_OK) {
             list_ms = ms;
             list = code;
+            cudaMemcpyAsync(&listed, a.list_count, sizeof(listed), cudaMemcpyDeviceToHost, ctx->stream);
             cudaMemsetAsync(a.list_count, 0, sizeof(unsigned int), ctx->stream);
             count_listed_kernel<<<1, 1024, 0, ctx->stream>>>(
                 a.uni_in, (int)tiles_of(variant(prec, code & (kTmaBit - 1)), a), a.list_count);
@@ -413,7 +418,10 @@ bsn_status stage_autotune(bsn_ctx* ctx, int prec, const f64::StageArgs& probe, d
         use.list = list;
         use.list_won = best & kListBit;
         const float tiles = (float)tiles_of(variant(prec, list & (kTmaBit - 1)), probe);
-        use.left_out = -1.f;
+        // of the timed stage; a small share may be gone by the last stage of the
+        // step, and is taken from the first count then
+        use.left_out = 1.f - (float)listed / tiles;
+        if (use.left_out < 0.3f) use.left_out = -1.f;
         use.no_gain = use.list_won ? 0.f : 1.f - (float)mixed / tiles;
         use.taken_at = 0.f;
         use.calls = 0;

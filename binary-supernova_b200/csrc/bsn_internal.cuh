@@ -45,7 +45,7 @@ struct bsn_ctx {
     std::set<std::pair<int, int>> settled;
     // steps that may list uniform tiles (autotune.cu): the fastest choice
     // without and with a list, whether the list was faster when they were timed
-    // and the share of tiles it then left out (below 0: not known yet), the
+    // and the share of tiles it then left out (below 0: the first count tells), the
     // share of uniform tiles up to which it is known not to pay, the one it was
     // last taken up at, and where later counts arrive: a word of pinned memory
     // (none for grids past the array's end)
